@@ -967,7 +967,7 @@ struct Ctx : pgdg_ctx {
     }
     timed("iface_gather", 6, [&] { Launch<D, R, EX>::iface_gather(K, P, Q, st); });
     int rc = PGDG_OK;
-    timed("mgfm_seeded", net ? 8 : 6, [&] {
+    timed("mgfm_seeded", net ? 3 : 1, [&] {
       rc = mgfm_seeded_run(net, Q.in6, Q.mat, d_gam, d_pinf, K.mgfm_variant, Q.out3, nullptr, Q.cap,
                            &P.cnt->mgfm_calls, part, st, Q.tot + 1);
     });

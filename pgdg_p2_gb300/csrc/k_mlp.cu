@@ -51,7 +51,8 @@ __host__ __device__ inline double mgfm_baseline(double ul, double ur, double pl,
   if (!(p0 > 1e-8)) p0 = 1e-8;
   const double Wl = sqrt(0.5 * rl * ((gl + 1.) * p0 + (gl - 1.) * pl + 2. * gl * il));
   const double Wr = sqrt(0.5 * rr * ((gr + 1.) * p0 + (gr - 1.) * pr + 2. * gr * ir));
-  double pt = (pl / Wl + pr / Wr + (ul - ur)) / (1. / Wl + 1. / Wr);
+  const double yl = drcp(Wl), yr = drcp(Wr);
+  double pt = (ddiv_by(pl, Wl, yl) + ddiv_by(pr, Wr, yr) + (ul - ur)) / (yl + yr);
   if (!(pt > 1e-8)) pt = 1e-8;
   return pt;
 }
@@ -79,19 +80,20 @@ __host__ __device__ inline void mgfm_features(const double* q, double gl, double
   const float a0 = sqrtf((float)P0 / sqrtf((float)rl * (float)rr));
   const float du = (float)(ul - ur) / a0;
   const double pb = mgfm_baseline(ul, ur, pl, pr, rl, rr, gl, il, gr, ir);
+  const double y0 = drcp(P0); /* six quotients by P0 */
   const float lbl = logf((float)(pb / pl)), lbr = logf((float)(pb / pr));
   const float sv = fabsf(lbl) + fabsf(lbr);
-  x[0] = logf((float)(Pl / P0));
-  x[1] = logf((float)(Pr / P0));
+  x[0] = logf((float)ddiv_by(Pl, P0, y0));
+  x[1] = logf((float)ddiv_by(Pr, P0, y0));
   x[2] = logf((float)(rl / rr));
   x[3] = du > 20.f ? 20.f : (du < -20.f ? -20.f : du);
   x[4] = lbl;
   x[5] = (float)gl;
   x[6] = (float)gr;
-  x[7] = (float)(il / P0);
-  x[8] = (float)(ir / P0);
-  x[9] = logf((float)(pl / P0 + 1e-30));
-  x[10] = logf((float)(pr / P0 + 1e-30));
+  x[7] = (float)ddiv_by(il, P0, y0);
+  x[8] = (float)ddiv_by(ir, P0, y0);
+  x[9] = logf((float)(ddiv_by(pl, P0, y0) + 1e-30));
+  x[10] = logf((float)(ddiv_by(pr, P0, y0) + 1e-30));
   x[11] = lbr;
   *pb_out = pb;
   *sc_out = sv * sv / (1.f + sv * sv);
@@ -367,43 +369,16 @@ __global__ void k_seed_features(const double* __restrict__ in6, const int8_t* __
   }
 }
 
-/* partition of a batch by the existence of a positive root: a problem without
- * one runs the plain Newton solve down to the 1e-8 floor (about 30 iterations)
- * while a seeded one converges in two or three, so the two kinds are solved in
- * separate warps.  flag[i] = 1 for a problem with a root (pb > 0 when the seed
- * path computed it, else f(1e-8) >= 0 evaluated here). */
-__global__ void k_root_flag(const double* __restrict__ in6, const int8_t* __restrict__ mat2,
-                            const double* __restrict__ gam, const double* __restrict__ pinf, int variant,
-                            const double* __restrict__ pb, unsigned long long* __restrict__ flag, int64_t n,
-                            const unsigned long long* __restrict__ dn) {
-  if (dn && (int64_t)*dn < n) n = (int64_t)*dn;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    bool root;
-    if (pb) {
-      root = pb[i] > 0;
-    } else {
-      const double* q = in6 + 6 * i;
-      const int s = mat2[2 * i], s1 = mat2[2 * i + 1];
-      double pl = q[2], pr = q[3], rl = q[4], rr = q[5];
-      if (variant == 0) {
-        pl = amax1(pl, 1e-10);
-        pr = amax1(pr, 1e-10);
-        rl = amax1(rl, 1e-10);
-        rr = amax1(rr, 1e-10);
-      } else {
-        if (pl < 0) pl = 0;
-        if (pr < 0) pr = 0;
-      }
-      root = !(mgfm_f(q[0], q[1], pl, pr, rl, rr, gam[s], pinf[s], gam[s1], pinf[s1], 1e-8) < 0);
-    }
-    flag[i] = root ? 1ull : 0ull;
-  }
+/* partition of a seeded batch by the existence of a positive root (pb > 0):
+ * flag[i] = 1 for a problem with a root */
+__global__ void k_root_flag(const double* __restrict__ pb, unsigned long long* __restrict__ flag, int64_t n) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    flag[i] = pb[i] > 0 ? 1ull : 0ull;
 }
 /* order: problems with a root first, then the others, each in input order;
  * pos is the exclusive prefix of the flags, nroot_p their total */
 __global__ void k_root_perm(const unsigned long long* __restrict__ pos, const unsigned long long* __restrict__ nroot_p,
-                            int32_t* __restrict__ perm, int64_t n, const unsigned long long* __restrict__ dn) {
-  if (dn && (int64_t)*dn < n) n = (int64_t)*dn;
+                            int32_t* __restrict__ perm, int64_t n) {
   const int64_t nroot = (int64_t)*nroot_p;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t p = (int64_t)pos[i];
@@ -411,6 +386,14 @@ __global__ void k_root_perm(const unsigned long long* __restrict__ pos, const un
     perm[root ? p : nroot + (i - p)] = (int32_t)i;
   }
 }
+
+/* Threads per block of the FP64 kernels of the batched solve of n problems.  An
+ * FP64 instruction occupies a quarter of an SM for 64 cycles a warp, so the time of a
+ * batch that is resident at once is the largest number of warps on any quarter, and
+ * blocks of 64 spread it evenly; a larger batch wants all 2048 threads of an SM,
+ * which the capped grid reaches with blocks of 256 (1000 problems: 86 us with 64,
+ * 130 with 256; 65537: 228 and 257; 2^22: 13.1 ms and 11.8). */
+inline int newton_threads(int64_t n) { return n <= 152 * 1024 ? 64 : 256; }
 
 /* Newton from the seed (or the plain seed when seed is NULL or the entry is
  * negative); a seeded solve that has not converged at the cap is redone from
@@ -447,7 +430,8 @@ __global__ void k_mgfm_seeded(const double* __restrict__ in6, const int8_t* __re
        * early); otherwise the problem is solved again from the plain seed */
       done = it < 50 && isfinite(o[0]) && isfinite(o[1]) && isfinite(o[2]);
     }
-    if (!done) it += mgfm(q[0], q[1], q[2], q[3], q[4], q[5], gam[s], pinf[s], gam[s1], pinf[s1], variant, -1.0, o);
+    if (!done) it += mgfm(q[0], q[1], q[2], q[3], q[4], q[5], gam[s], pinf[s], gam[s1], pinf[s1], variant, -1.0, o,
+                           seed && sd <= 0 ? 1 : 0);
     out3[3 * i + 0] = o[0];
     out3[3 * i + 1] = o[1];
     out3[3 * i + 2] = o[2];
@@ -668,16 +652,10 @@ int pgdg_mgfm_batched(const pgdg_mlp* net, const double* in6, const int8_t* mat2
                       const double* pinf, int nmat, int variant, double* out3, int32_t* iters, int64_t n) {
   if (n < 0 || !in6 || !mat2 || !gam || !pinf || !out3 || nmat < 1) return PGDG_EINVAL;
   if (n == 0) return PGDG_OK;
-  /* partition scratch: the network's, or (plain seed) a per-device cache used
-   * under a lock; calls run on the default stream */
-  if (net) return mgfm_seeded_run((void*)net, in6, mat2, gam, pinf, variant, out3, iters, n, nullptr,
-                                  const_cast<pgdg_mlp*>(net)->part, 0, nullptr);
-  static PartScratch cache[64];
-  static std::mutex mu;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return PGDG_ECUDA;
-  std::lock_guard<std::mutex> lk(mu);
-  return mgfm_seeded_run(nullptr, in6, mat2, gam, pinf, variant, out3, iters, n, nullptr, cache[dev], 0, nullptr);
+  /* the partition scratch is the network's; plain solves need none */
+  PartScratch none;
+  return mgfm_seeded_run((void*)net, in6, mat2, gam, pinf, variant, out3, iters, n, nullptr,
+                         net ? const_cast<pgdg_mlp*>(net)->part : none, 0, nullptr);
 }
 
 /* Seeds of pgdg_mgfm_batched_noalloc: a file-scope device array, so the call
@@ -711,7 +689,7 @@ int pgdg_mgfm_batched_noalloc(const pgdg_mlp* net, const double* in6, const int8
     seed_launch(const_cast<pgdg_mlp*>(net), in6, mat2, gam, pinf, variant, seeds, n, 0);
     sd = seeds;
   }
-  k_mgfm_seeded<<<g_for(n, 256), 256>>>(in6, mat2, gam, pinf, variant, sd, out3, iters, n, nullptr, nullptr, nullptr,
+  k_mgfm_seeded<<<g_for(n, newton_threads(n)), newton_threads(n)>>>(in6, mat2, gam, pinf, variant, sd, out3, iters, n, nullptr, nullptr, nullptr,
                                         nullptr, nullptr, nullptr, nullptr);
   return cudaGetLastError() == cudaSuccess ? PGDG_OK : PGDG_ECUDA;
 }
@@ -747,9 +725,8 @@ void PartScratch::release() {
 }
 
 int mgfm_seeded_reserve(void* netv, PartScratch& ps, int64_t n) {
-  int rc = ps.reserve(n);
-  if (rc == PGDG_OK && netv) rc = static_cast<pgdg_mlp*>(netv)->reserve_seeds(n);
-  return rc;
+  (void)ps; /* a stage's batch is not sorted */
+  return netv ? static_cast<pgdg_mlp*>(netv)->reserve_seeds(n) : PGDG_OK;
 }
 
 int mgfm_seeded_run(void* netv, const double* in6, const int8_t* mat2, const double* gam, const double* pinf,
@@ -758,31 +735,39 @@ int mgfm_seeded_run(void* netv, const double* in6, const int8_t* mat2, const dou
   if (n <= 0) return PGDG_OK;
   if (n > INT32_MAX) return PGDG_EINVAL;
   pgdg_mlp* m = static_cast<pgdg_mlp*>(netv);
-  int rc = ps.reserve(n);
-  if (rc) return rc;
   const double* sd = nullptr;
   if (m) {
     /* split seed path: features and baseline, the network, then Newton with the
      * seed formed per problem (same arithmetic as the fused k_seed) */
-    rc = m->reserve_seeds(n);
+    const int rc = m->reserve_seeds(n);
     if (rc) return rc;
-    k_seed_features<<<g_for(n, 256), 256, 0, st>>>(in6, mat2, gam, pinf, variant, m->Xb, m->seeds, m->sc, n, dn);
+    k_seed_features<<<g_for(n, newton_threads(n)), newton_threads(n), 0, st>>>(in6, mat2, gam, pinf, variant, m->Xb, m->seeds, m->sc, n, dn);
     forward(m, m->Xb, m->Yb, nullptr, nullptr, nullptr, n, st, dn);
     sd = m->seeds;
   }
-  /* problems with a root first: warps of converging problems are not held up
-   * by the long floor descent of problems without one (results per problem
-   * are unchanged) */
-  if (!dn) {
-    const unsigned long long nn = (unsigned long long)n;
-    cudaMemcpyAsync(ps.dn, &nn, sizeof(nn), cudaMemcpyHostToDevice, st);
+  /* A problem without a root takes about as long as one with a root from the plain
+   * seed (mgfm replays its descent), so plain solves are one launch: 2^22 problems
+   * 17.3 -> 11.8 ms, 65537 problems 550 -> 255 us.  Seeded, it takes about six
+   * iterations and the others two, and a batch is sorted, problems with a root
+   * first: 2^22 problems 10.9 -> 5.9 ms; at 65537 217 us sorted and 242 unsorted, at
+   * 1000 111 and 103.  A stage of a run (dn) is not sorted: nearly all its problems
+   * have a root. */
+  const bool sorted = m && !dn && n > 16384;
+  if (!sorted) {
+    k_mgfm_seeded<<<g_for(n, newton_threads(n)), newton_threads(n), 0, st>>>(in6, mat2, gam, pinf, variant, sd, out3, iters, n, stats,
+                                                 m ? m->Yb : nullptr, m ? m->sc : nullptr, m ? m->d_params : nullptr,
+                                                 nullptr, m && m->tc ? m->d_tcerr : nullptr, dn);
+    return cudaGetLastError() == cudaSuccess ? PGDG_OK : PGDG_ECUDA;
   }
-  k_root_flag<<<g_for(n, 256), 256, 0, st>>>(in6, mat2, gam, pinf, variant, sd, ps.pos, n, dn);
-  scan_u64(ps.pos, ps.blk, dn ? dn : ps.dn, n, st);
-  k_root_perm<<<g_for(n, 256), 256, 0, st>>>(ps.pos, ps.blk + (n + 2047) / 2048, ps.perm, n, dn);
-  k_mgfm_seeded<<<g_for(n, 256), 256, 0, st>>>(in6, mat2, gam, pinf, variant, sd, out3, iters, n, stats,
-                                               m ? m->Yb : nullptr, m ? m->sc : nullptr, m ? m->d_params : nullptr,
-                                               ps.perm, m && m->tc ? m->d_tcerr : nullptr, dn);
+  const int rc = ps.reserve(n);
+  if (rc) return rc;
+  const unsigned long long nn = (unsigned long long)n;
+  cudaMemcpyAsync(ps.dn, &nn, sizeof(nn), cudaMemcpyHostToDevice, st);
+  k_root_flag<<<g_for(n, 256), 256, 0, st>>>(sd, ps.pos, n);
+  scan_u64(ps.pos, ps.blk, ps.dn, n, st);
+  k_root_perm<<<g_for(n, 256), 256, 0, st>>>(ps.pos, ps.blk + (n + 2047) / 2048, ps.perm, n);
+  k_mgfm_seeded<<<g_for(n, newton_threads(n)), newton_threads(n), 0, st>>>(in6, mat2, gam, pinf, variant, sd, out3, iters, n, stats,
+                                               m->Yb, m->sc, m->d_params, ps.perm, m->tc ? m->d_tcerr : nullptr, nullptr);
   return cudaGetLastError() == cudaSuccess ? PGDG_OK : PGDG_ECUDA;
 }
 }  // namespace pgdg

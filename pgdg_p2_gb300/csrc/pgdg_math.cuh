@@ -129,19 +129,60 @@ PGDG_HD double wl_cal(double rhol, double pl, double ps, double g, double pinf) 
   double in = dadd(dadd(dmul(dadd(g, 1.0), ps), dmul(dsub(g, 1.0), pl)), dmul(dmul(2.0, g), pinf));
   return dsqrt(dmul(dmul(0.5, rhol), in));
 }
-PGDG_HD double jaco_cal(double W, double pl, double rhol, double ps, double g) {
-  double t = ddiv(dsub(ps, pl), dmul(W, W));
+/* 1 / b correctly rounded */
+PGDG_HD double drcp(double b) {
+#if defined(__CUDA_ARCH__)
+  return __drcp_rn(b);
+#else
+  return ddiv(1.0, b);
+#endif
+}
+/* a / b correctly rounded, given y = 1 / b correctly rounded: a quotient from y,
+ * corrected twice by its exact remainder (Markstein, IBM J. Res. Dev. 34, 1990:
+ * with y correctly rounded and a quotient within one unit in the last place, the
+ * corrected quotient is the correctly rounded one).  5 FP64 instructions where
+ * a division is about 10 and the FP64 pipe sets the pace.  Outside exponents
+ * that keep every step normal, and for b <= 0, the division itself. */
+PGDG_HD double ddiv_by(double a, double b, double y) {
+#if defined(__CUDA_ARCH__)
+  const int ha = __double2hiint(a) & 0x7fffffff;
+  const unsigned ea = (unsigned)ha >> 20, eb = (unsigned)__double2hiint(b) >> 20;
+  if ((ea - 400u < 1200u || (ha | __double2loint(a)) == 0) && eb - 600u < 800u) { /* a sign bit in b fails the range too */
+    double q = __dmul_rn(a, y);
+    q = __fma_rn(__fma_rn(-q, b, a), y, q);
+    return __fma_rn(__fma_rn(-q, b, a), y, q);
+  }
+#endif
+  return ddiv(a, b);
+}
+
+/* d/dp of (p - p0) / W(p), with d = p - p0 and y = 1 / W; d / W^2 rho (g + 1) / 4 / W
+ * keeps the reference's order (the quarter is exact) */
+PGDG_HD double jaco_cal(double W, double y, double d, double rhol, double g) {
+  double t = ddiv(d, dmul(W, W));
   t = dmul(t, rhol);
   t = dmul(t, dadd(g, 1));
-  t = ddiv(t, 4.);
-  t = ddiv(t, W);
-  return dsub(ddiv(1., W), t);
+  t = dmul(t, 0.25);
+  t = ddiv_by(t, W, y);
+  return dsub(y, t);
 }
 
 /* Two-shock Newton solve; variant 0 = mpm.cpp:882-926, 1 = Triple_point_2phase/
- * mpm.cpp:1373-1416.  seed_p > 0 replaces the initial p*.  Returns iterations. */
+ * mpm.cpp:1373-1416.  seed_p > 0 replaces the initial p*.  Returns iterations.
+ *
+ * A problem without a positive root: f(p) = u_l - u_r - (p - p_l) / W_l -
+ * (p - p_r) / W_r falls and is convex, so f(1e-8) >= f(p) + |f'(p)| (p - 1e-8).  With
+ * f(1e-8) < 0 Newton's step |f / f'| is longer than p - 1e-8, so the cap 0.6 p decides
+ * it for every p > 2.5e-8; and |f(p)| >= |f(1e-8)|, so with f(1e-8) below the
+ * tolerance no iterate on the way converges.  The iterates down to 4e-8 are then
+ * p - 0.6 p, two operations in place of about 130, and the rest runs as usual: the
+ * same bits and counts.  descent = 1 looks for this at once (the caller knows
+ * that f(1e-8) < 0), 0 after two capped steps downwards; DESCENT = false leaves it
+ * out (the residual's inline solves converge in two or three iterations, and the
+ * registers count there). */
+template <bool DESCENT = true>
 PGDG_HD int mgfm(double ul, double ur, double pl, double pr, double rhol, double rhor, double gl,
-                 double pinfl, double gr, double pinfr, int variant, double seed_p, double out[3]) {
+                 double pinfl, double gr, double pinfr, int variant, double seed_p, double out[3], int descent = 0) {
   double pstar;
   if (variant == 0) {
     pl = amax1(pl, 1e-10);
@@ -155,21 +196,37 @@ PGDG_HD int mgfm(double ul, double ur, double pl, double pr, double rhol, double
     pstar = dmul(dadd(pl, pr), 0.5);
   }
   if (seed_p > 0) pstar = seed_p;
-  double tol = amax1(1e-8, dmul(1e-3, fabs(dsub(ul, ur))));
-  double f1 = 1.;
-  double rhols = 0, usl = 0, Wl = 0, Wr = 0;
-  int nn = 0;
+  const double du = dsub(ul, ur);
+  const double tol = amax1(1e-8, dmul(1e-3, fabs(du)));
+  double f1 = 1., Wl = 0, ql = 0, pold = pstar, usl;
+  int nn = 0, down = descent ? 2 : 0;
   do {
+    if (DESCENT && down == 2) {
+      down = 3; /* looked at once */
+      /* the convexity above holds for these; the margins cover the rounding of f */
+      if (pstar > 4e-8 && pstar < 1e100 && rhol > 0 && rhor > 0 && gl > 1 && gr > 1 && pinfl >= 0 && pinfr >= 0) {
+        const double f0 = dsub(dsub(du, ddiv(dsub(1e-8, pl), wl_cal(rhol, pl, 1e-8, gl, pinfl))),
+                               ddiv(dsub(1e-8, pr), wl_cal(rhor, pr, 1e-8, gr, pinfr)));
+        if (f0 < dmul(-1.001, tol) && f0 > -1e100)
+          while (pstar > 4e-8 && nn < 48) {
+            pstar = dsub(pstar, dmul(0.6, pstar));
+            nn++;
+          }
+      }
+    }
     Wl = wl_cal(rhol, pl, pstar, gl, pinfl);
-    Wr = wl_cal(rhor, pr, pstar, gr, pinfr);
-    if (variant == 0) usl = dsub(ul, ddiv(dsub(pstar, pl), Wl));
-    rhols = rhols_cal(rhol, pl, pstar, gl, pinfl);
-    f1 = dsub(dsub(dsub(ul, ur), ddiv(dsub(pstar, pl), Wl)), ddiv(dsub(pstar, pr), Wr));
-    double jac = dsub(-jaco_cal(Wl, pl, rhol, pstar, gl), jaco_cal(Wr, pr, rhor, pstar, gr));
+    const double Wr = wl_cal(rhor, pr, pstar, gr, pinfr);
+    const double yl = drcp(Wl), yr = drcp(Wr), dl = dsub(pstar, pl), dr = dsub(pstar, pr);
+    ql = ddiv_by(dl, Wl, yl);
+    f1 = dsub(dsub(du, ql), ddiv_by(dr, Wr, yr));
+    const double jac = dsub(-jaco_cal(Wl, yl, dl, rhol, gl), jaco_cal(Wr, yr, dr, rhor, gr));
     double dp = ddiv(-f1, jac);
-    double cap = dmul(0.6, pstar);
-    if (fabs(dp) > cap) dp = copysign(cap, dp);
-    const double pold = pstar;
+    const double cap = dmul(0.6, pstar);
+    if (fabs(dp) > cap) {
+      dp = copysign(cap, dp);
+      if (dp < 0 && down < 2) down++;
+    }
+    pold = pstar;
     pstar = dadd(pstar, dp);
     pstar = amax1(pstar, 1e-8);
     nn++;
@@ -182,8 +239,10 @@ PGDG_HD int mgfm(double ul, double ur, double pl, double pr, double rhol, double
       break;
     }
   } while (fabs(f1) > tol && nn < 50);
-  if (variant != 0) usl = dsub(ul, ddiv(dsub(pstar, pl), Wl));
-  out[0] = rhols;
+  /* the density and (variant 0) the velocity of the last iterate evaluated */
+  if (variant == 0) usl = dsub(ul, ql);
+  else usl = dsub(ul, ddiv(dsub(pstar, pl), Wl));
+  out[0] = rhols_cal(rhol, pl, pold, gl, pinfl);
   out[1] = pstar;
   out[2] = usl;
   return nn;

@@ -278,8 +278,9 @@ struct Ctx : pgdg_ctx {
     CK(A(&P.cnt, 1));
     CK(A(&d_tot, Launch<D, R, EX>::totals_scratch()));
     /* interface queue: at most 2 phases x 2D faces x 4 points x 1 other phase per cell;
-     * sized for a few per cent of the cells, grown on demand */
-    Q.cap = std::max<int64_t>(1 << 16, K.ncell / 8);
+     * sized for a few per cent of the cells, grown on demand when the queue was asked
+     * for (a stage that outgrows it is solved inline) */
+    Q.cap = std::max<int64_t>(1 << 16, sizeof(R) == 8 ? K.ncell : K.ncell / 8);
     CK(A(&Q.in6, 6 * (size_t)Q.cap));
     CK(A(&Q.mat, 2 * (size_t)Q.cap));
     CK(A(&Q.out3, 3 * (size_t)Q.cap));
@@ -954,14 +955,20 @@ struct Ctx : pgdg_ctx {
     return PGDG_OK;
   }
   int grid_acc() override {
-    if (!iface_queue || EX) {
+    /* FP32 residual without the queue: solved inline, as its rounding differs
+     * between the inline and the queued build */
+    if (!iface_queue && sizeof(R) == 4) {
       timed("grid_acc", 1, [&] { Launch<D, R, EX>::grid_acc(K, P, st); });
       return PGDG_OK;
     }
-    /* surrogate-seeded MGFM: queue the interface problems, solve them in one
-     * batch, then evaluate the residual with the queued ghost states.  The
-     * batch's size stays on the device (Q.tot): nothing is read back */
-    if (!capturing) {
+    /* queue the interface problems, solve them in one batch (from the surrogate's
+     * seeds when one is attached), then evaluate the residual with the queued
+     * ghost states.  On the FP64 paths also without a surrogate: an interface cell
+     * would solve up to 2 F x 2D faces x points one after another, its warp
+     * waiting at 64 cycles an FP64 instruction (exact path, 48x12x12 cells: residual
+     * 4.4 -> 3.6 ms per step, the same bits).  The batch's size stays on the device
+     * (Q.tot): nothing is read back */
+    if (iface_queue && !capturing) {
       const int rc = mgfm_seeded_reserve(net, part, Q.cap);
       if (rc) return rc;
     }
@@ -993,7 +1000,9 @@ struct Ctx : pgdg_ctx {
       if (xn == xs || xn == x0 || xn < 0 || xn > 2) xn = (xs + 1) % 3;  /* md 1 without md 0 */
     }
     timed("g2p", 1, [&] { Launch<D, R, EX>::g2p(K, P, md, xs, x0, xn, hn, !g2p_partial, st); });
-    if (!EX) timed("rowsort", 3, [&] { Launch<D, R, EX>::rowsort(K, P, xs, pst_scratch, st); });
+    /* (variant 8 of the FP64 path scans the cells and reads no sorted rows) */
+    if (!EX && !(sizeof(R) == 8 && pst_var == 8))
+      timed("rowsort", 3, [&] { Launch<D, R, EX>::rowsort(K, P, xs, pst_scratch, st); });
     if (pst_var < 0)
       pst_var = tune(Launch<D, R, EX>::pst_variants(),
                      [&](int v) { Launch<D, R, EX>::pst(K, P, xs, hs, xn, hn, v, pst_scratch, st); });

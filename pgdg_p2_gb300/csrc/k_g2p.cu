@@ -185,9 +185,8 @@ void Launch<D, R, EX>::g2p(const CaseK& K, const DevPtrs<R>& P, int md, int xs, 
  *     Each thread then takes one particle: per row, a binary search finds the
  *     chord of its 2h sphere, the cell tag keeps the reference's +-rad2 window,
  *     and members are summed at once (or queued, variant 0) in sorted order.
- *   - Exact path: per-cell list offsets, the exact bounding box of each cell's
- *     entries and the reference's list order (binned entries, boundary
- *     particles, appended entries), scanned cell by cell.
+ *   - Exact path: k_pst_d below, which scans cell by cell in the reference's list
+ *     order (binned entries, boundary particles, appended entries).
  * A particle whose scan range leaves the staged box (it crossed a cell face
  * during the first stage) reads global memory instead, in the reference's list
  * order. */
@@ -243,17 +242,13 @@ struct RowKey;
 template <int D, typename R>
 struct PstSmem {
   using V4 = typename Vec4<R>::T;
-  int* off;      /* nsc + 1 */
-  int* mid;      /* nsc: index of the first appended entry of each staged cell */
   int* bnd;      /* nsc: cell holds boundary particles */
-  R* blo;        /* D * nsc */
-  R* bhi;        /* D * nsc */
   V4* ent;       /* cap: (x, y, z | slot) of each staged particle at the stage start */
   unsigned short* buf; /* PST_BUF x PST_THREADS queued member entries */
-  /* mixed / FMA paths: off holds per staged row (not per cell) the offsets of
-   * its entries, which are sorted by the last-axis coordinate (z in 3D, y in
-   * 2D); ecell holds each entry's cell offset in the row window, rlo/rhi the
-   * row's bounds in the other axes */
+  /* off holds per staged row the offsets of its entries, which are sorted by the
+   * last-axis coordinate (z in 3D, y in 2D); ecell holds each entry's cell offset
+   * in the row window, rlo/rhi the row's bounds in the other axes */
+  int* off;      /* nrow + 1 */
   unsigned char* ecell; /* cap */
   R* rlo;        /* 2 * nrow */
   R* rhi;        /* 2 * nrow */
@@ -262,7 +257,7 @@ struct PstSmem {
 };
 
 /* shared-memory layout of one brick; with sm == nullptr only the size */
-template <int D, typename R, bool EX>
+template <int D, typename R>
 __host__ __device__ inline size_t pst_layout(PstSmem<D, R>* sm, unsigned char* raw, int nsc, int nrow, int cap,
                                              int qdepth) {
   using V4 = typename Vec4<R>::T;
@@ -275,31 +270,22 @@ __host__ __device__ inline size_t pst_layout(PstSmem<D, R>* sm, unsigned char* r
   };
   const size_t off_o = take(sizeof(int) * (size_t)((nsc > nrow ? nsc : nrow) + 1), 16);
   const size_t bnd_o = take(sizeof(int) * (size_t)nsc, 16);
-  const size_t mid_o = EX ? take(sizeof(int) * (size_t)nsc, 16) : 0;
-  const size_t blo_o = EX ? take(sizeof(R) * (size_t)(2 * D * nsc), 16) : 0;
   const size_t ent_o = take(sizeof(V4) * (size_t)cap, 32);
   const size_t buf_o = take(sizeof(unsigned short) * (size_t)qdepth * PST_THREADS, 16);
-  const size_t rlo_o = EX ? 0 : take(sizeof(R) * (size_t)(4 * nrow), 16);
-  const size_t ec_o = EX ? 0 : take((size_t)cap, 16);
-  const size_t rs_o = EX ? 0 : take(sizeof(long long) * (size_t)nrow, 16);
+  const size_t rlo_o = take(sizeof(R) * (size_t)(4 * nrow), 16);
+  const size_t ec_o = take((size_t)cap, 16);
+  const size_t rs_o = take(sizeof(long long) * (size_t)nrow, 16);
   if (sm) {
     sm->off = reinterpret_cast<int*>(raw + off_o);
     sm->bnd = reinterpret_cast<int*>(raw + bnd_o);
-    sm->mid = EX ? reinterpret_cast<int*>(raw + mid_o) : nullptr;
-    sm->blo = EX ? reinterpret_cast<R*>(raw + blo_o) : nullptr;
-    sm->bhi = EX ? sm->blo + D * nsc : nullptr;
     sm->ent = reinterpret_cast<V4*>(raw + ent_o);
     sm->buf = reinterpret_cast<unsigned short*>(raw + buf_o);
-    sm->rlo = EX ? nullptr : reinterpret_cast<R*>(raw + rlo_o);
-    sm->rhi = EX ? nullptr : sm->rlo + 2 * nrow;
-    sm->ecell = EX ? nullptr : raw + ec_o;
-    sm->rsrc = EX ? nullptr : reinterpret_cast<long long*>(raw + rs_o);
+    sm->rlo = reinterpret_cast<R*>(raw + rlo_o);
+    sm->rhi = sm->rlo + 2 * nrow;
+    sm->ecell = raw + ec_o;
+    sm->rsrc = reinterpret_cast<long long*>(raw + rs_o);
   }
   return o + 128;
-}
-template <int D, typename R, bool EX>
-__device__ inline void pst_carve(PstSmem<D, R>& sm, unsigned char* raw, int qdepth) {
-  pst_layout<D, R, EX>(&sm, raw, sm.nsc, sm.nrow, sm.cap, qdepth);
 }
 
 /* per-particle constants and accumulators of the shifting sum */
@@ -307,6 +293,7 @@ template <int D, typename R, bool EX>
 struct PstPart {
   R xsp[3], xnp[3];
   R hs_p, hh, lim2, rho_p, c_p, crho_p, tmp1c, C, W_dp, inv_hh, inv_wdp, aw_c, cwr, tmp1c5;
+  R m5c; /* -5 C (exact path) */
   int ph;
   R pst[3], phs[3];
 
@@ -328,6 +315,7 @@ struct PstPart {
     aw_c = R(-5.) * C * inv_hh * inv_hh; /* dW/dr / r = -5 C q^3 / h^2 */
     cwr = C * inv_wdp;
     tmp1c5 = R(0.2) * tmp1c;
+    m5c = R(-5.) * C;
     for (int d = 0; d < 3; d++) pst[d] = phs[d] = R(0);
   }
 
@@ -381,17 +369,18 @@ struct PstPart {
       }
       return;
     }
-    /* exact path: the reference's operation order */
+    /* exact path: the reference's operation order, with the quotients by h and
+     * W_dp from their correctly rounded reciprocals (inv_hh, inv_wdp; the same bits) */
     R s, q, q3, Wij, aw, rr;
     {
       R dist = sqrt_r<R>(d2);
-      s = dist / hh;
+      s = ddiv_by(dist, hh, inv_hh);
       if (!(s < R(2))) return; /* W and dW vanish beyond the support */
       q = R(1.) - R(0.5) * s;
       q3 = (q * q) * q;
       Wij = C * (q3 * q) * (R(1.) + R(2.) * s);
-      aw = R(-5.) * C * q3 * s / hh / dist;
-      rr = Wij / W_dp;
+      aw = ddiv_by(m5c * q3 * s, hh, inv_hh) / dist;
+      rr = ddiv_by(Wij, W_dp, inv_wdp);
     }
     R Rr = R(0.2) * ((rr * rr) * (rr * rr));
     R tmp1 = tmp1c * (R(1) + Rr);
@@ -1078,34 +1067,6 @@ __device__ void pst_particle(const CaseK& K, const DevPtrs<R>& P, int64_t p, con
               const int64_t c = ((int64_t)t * K.N[1] + s) * K.N[2] + m;
               pst_boundary_cell<D, R, EX>(K, P, c, pp);
             }
-    } else {
-      /* exact path: the reference's per-cell list order (binned fluid,
-       * boundary particles, appended fluid) */
-      for (int t = lo[0]; t <= hi[0]; t++)
-        for (int s = lo[1]; s <= hi[1]; s++) {
-          int l = ((t - sm->lo[0]) * sm->n[1] + (s - sm->lo[1])) * sm->n[2] + (lo[2] - sm->lo[2]);
-          for (int m = lo[2]; m <= hi[2]; m++, l++) {
-            const int e0 = sm->off[l], e1 = sm->off[l + 1], em = e0 + sm->mid[l];
-            R md = R(0);
-            for (int d = 0; d < D; d++) {
-              R a = sm->blo[d * sm->nsc + l] - pp.xsp[d];
-              R b = pp.xsp[d] - sm->bhi[d * sm->nsc + l];
-              R g = a > b ? a : b;
-              if (g > R(0)) md += g * g;
-            }
-            if (md <= lim2m)
-              for (int e = e0; e < em; e++) queue(e);
-            if (sm->bnd[l]) {
-              flush();
-              const int64_t c = ((int64_t)t * K.N[1] + s) * K.N[2] + m;
-              pst_boundary_cell<D, R, EX>(K, P, c, pp);
-            }
-            if (md <= lim2m)
-              for (int e = em; e < e1; e++) queue(e);
-            if (__any_sync(__activemask(), nbuf >= BUFV / 2)) flush();
-          }
-        }
-      flush();
     }
   } else {
     for (int t = lo[0]; t <= hi[0]; t++)
@@ -1134,7 +1095,7 @@ __device__ void pst_particle(const CaseK& K, const DevPtrs<R>& P, int64_t p, con
   pst_finish<D, R, EX>(K, P, p, dt, pp);
 }
 
-template <int D, typename R, bool EX, int VAR>
+template <int D, typename R, int VAR>
 __global__ void __launch_bounds__(pst_threads(VAR), pst_minblocks(VAR)) k_pst(CaseK K, DevPtrs<R> P, int xs, int hs, int xn, int hn,
                                                     int nb0, int nb1, int cap, RowSorted<R> RS) {
   using BK = BrickOf<D, VAR>;
@@ -1165,21 +1126,10 @@ __global__ void __launch_bounds__(pst_threads(VAR), pst_minblocks(VAR)) k_pst(Ca
   sm.nsc = sm.n[0] * sm.n[1] * sm.n[2];
   sm.cap = cap;
   sm.nrow = (D == 3) ? sm.n[0] * sm.n[1] : sm.n[0];
-  pst_carve<D, R, EX>(sm, smem_raw, (!EX && pst_direct(VAR)) ? 0 : PST_BUF);
+  pst_layout<D, R>(&sm, smem_raw, sm.nsc, sm.nrow, sm.cap, pst_direct(VAR) ? 0 : PST_BUF);
   __shared__ int s_red[SCAN_RED];
   int s_total;
-  if constexpr (EX) {
-    for (int l = threadIdx.x; l < sm.nsc; l += blockDim.x) {
-      int t = l / (sm.n[1] * sm.n[2]), s = (l / sm.n[2]) % sm.n[1], m = l % sm.n[2];
-      int64_t c = ((int64_t)(sm.lo[0] + t) * K.N[1] + (sm.lo[1] + s)) * K.N[2] + (sm.lo[2] + m);
-      int cnt = min(P.bcnt[c], K.maxpc);
-      sm.off[l + 1] = cnt;
-      sm.mid[l] = cnt;
-      sm.bnd[l] = P.boff[c + 1] > P.boff[c] ? 1 : 0;
-    }
-    __syncthreads();
-    s_total = block_scan_counts(sm.off, sm.nsc, s_red);
-  } else {
+  {
     /* boundary-particle flag of each staged cell, and per staged row the range
      * of the stage's row-sorted entries that holds every entry of the row's
      * window cells (entries of other cells of the row can lie inside the range
@@ -1208,54 +1158,7 @@ __global__ void __launch_bounds__(pst_threads(VAR), pst_minblocks(VAR)) k_pst(Ca
   }
   const bool use_sm = s_total <= cap;
   if (use_sm) {
-    if constexpr (EX) {
-      /* slots: one thread per staged cell copies its list into the entry
-       * slots and finds the first appended entry (the reference's list order
-       * puts the appended split children after the boundary particles) */
-      for (int l = threadIdx.x; l < sm.nsc; l += blockDim.x) {
-        const int t = l / (sm.n[1] * sm.n[2]), s = (l / sm.n[2]) % sm.n[1], m = l % sm.n[2];
-        const int64_t c = ((int64_t)(sm.lo[0] + t) * K.N[1] + (sm.lo[1] + s)) * K.N[2] + (sm.lo[2] + m);
-        const int32_t* bk = P.bucket + c * K.maxpc;
-        const int e0 = sm.off[l], cnt = sm.off[l + 1] - e0;
-        bool app = false;
-        for (int r = 0; r < cnt; r++) {
-          const int32_t q = bk[r];
-          sm.ent[e0 + r].w = slot_as<R>(q);
-          if (!app && P.lkey[q] >= KEY_APPEND) {
-            sm.mid[l] = r;
-            app = true;
-          }
-        }
-      }
-      __syncthreads();
-      /* stage-start coordinates: one thread per entry */
-      for (int e = threadIdx.x; e < s_total; e += blockDim.x) {
-        V4 v = sm.ent[e];
-        const int32_t q = slot_of<R>(v.w);
-        v.x = XS[q];
-        v.y = XS[K.cap + q];
-        v.z = (D == 3) ? XS[2 * K.cap + q] : R(0);
-        sm.ent[e] = v;
-      }
-      __syncthreads();
-      /* per cell: the exact bounding box of its entries */
-      for (int l = threadIdx.x; l < sm.nsc; l += blockDim.x) {
-        R mn[3] = {R(1e30), R(1e30), R(1e30)}, mx[3] = {R(-1e30), R(-1e30), R(-1e30)};
-        for (int e = sm.off[l]; e < sm.off[l + 1]; e++) {
-          const V4 v = sm.ent[e];
-          const R xv[3] = {v.x, v.y, v.z};
-          for (int d = 0; d < D; d++) {
-            mn[d] = xv[d] < mn[d] ? xv[d] : mn[d];
-            mx[d] = xv[d] > mx[d] ? xv[d] : mx[d];
-          }
-        }
-        for (int d = 0; d < D; d++) {
-          sm.blo[d * sm.nsc + l] = mn[d];
-          sm.bhi[d * sm.nsc + l] = mx[d];
-        }
-      }
-      __syncthreads();
-    } else {
+    {
       /* one warp per staged row copies its range (coalesced), tags each entry
        * with its cell's offset in the row window (255 outside the window) and
        * reduces the row's bounds in the other axes */
@@ -1319,11 +1222,11 @@ __global__ void __launch_bounds__(pst_threads(VAR), pst_minblocks(VAR)) k_pst(Ca
     }
     const int64_t c = s_bcell[q];
     const int32_t p = P.bucket[c * K.maxpc + (i - s_boff[q])];
-    pst_particle<D, R, EX, VAR>(K, P, p, XS, XN, HS, HN, dt, max_v, use_sm ? &sm : nullptr);
+    pst_particle<D, R, false, VAR>(K, P, p, XS, XN, HS, HN, dt, max_v, use_sm ? &sm : nullptr);
   }
 }
 
-template <int D, typename R, bool EX, int VAR>
+template <int D, typename R, int VAR>
 static void pst_launch(const CaseK& K, const DevPtrs<R>& P, int xs, int hs, int xn, int hn, const RowSorted<R>& RS,
                        cudaStream_t st) {
   using BK = BrickOf<D, VAR>;
@@ -1334,22 +1237,22 @@ static void pst_launch(const CaseK& K, const DevPtrs<R>& P, int xs, int hs, int 
   const int nsc = (BK::B0 + 2 * r) * (BK::B1 + 2 * r) * (D == 3 ? BK::B2 + 2 * r : 1);
   const int ppc = (D == 3) ? 8 : 4;
   const int nrow = (D == 3) ? (BK::B0 + 2 * r) * (BK::B1 + 2 * r) : (BK::B0 + 2 * r);
-  const int qdepth = (!EX && pst_direct(VAR)) ? 0 : PST_BUF;
+  const int qdepth = pst_direct(VAR) ? 0 : PST_BUF;
   /* staging headroom over the nominal count (split children); variant 3 keeps
    * it at 1/8 so three blocks fit in an SM's shared memory */
-  int cap = (!EX && (VAR == 3 || VAR >= 5)) ? nsc * ppc * 9 / 8 : nsc * ppc * 5 / 4;
+  int cap = (VAR == 3 || VAR >= 5) ? nsc * ppc * 9 / 8 : nsc * ppc * 5 / 4;
   if (cap > 65535) cap = 65535;
-  size_t bytes = pst_layout<D, R, EX>(nullptr, nullptr, nsc, nrow, cap, qdepth);
+  size_t bytes = pst_layout<D, R>(nullptr, nullptr, nsc, nrow, cap, qdepth);
   while (bytes > 220 * 1024 && cap > 256) {
     cap = cap * 3 / 4;
-    bytes = pst_layout<D, R, EX>(nullptr, nullptr, nsc, nrow, cap, qdepth);
+    bytes = pst_layout<D, R>(nullptr, nullptr, nsc, nrow, cap, qdepth);
   }
   static bool attr_set = false;
   if (!attr_set) {
-    cudaFuncSetAttribute(k_pst<D, R, EX, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+    cudaFuncSetAttribute(k_pst<D, R, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
     attr_set = true;
   }
-  k_pst<D, R, EX, VAR><<<nbx * nb1 * nb0, pst_threads(VAR), bytes, st>>>(K, P, xs, hs, xn, hn, nb0, nb1, cap, RS);
+  k_pst<D, R, VAR><<<nbx * nb1 * nb0, pst_threads(VAR), bytes, st>>>(K, P, xs, hs, xn, hn, nb0, nb1, cap, RS);
 }
 
 /* ---- the shifting kernel, second form (variants 6 and 7) ----
@@ -1727,6 +1630,288 @@ static void pst2_launch(const CaseK& K, const DevPtrs<R>& P, int xs, int hs, int
   k_pst2<D, R, SREC><<<nbx * nb1 * nb0, 512, bytes_for(cap), st>>>(K, P, xs, hs, xn, hn, nb0, nb1, cap, RS);
 }
 
+/* ---- the shifting kernel of the FP64 paths ----
+ * An FP64 instruction occupies a quarter of an SM for 64 cycles a warp, 32 times
+ * an FP32 one, so everything that only decides is done in FP32: positions are
+ * staged relative to the brick's centre as (x, y, z, slot) in 16 bytes, cells
+ * are pruned by their FP32 bounds, and a candidate is a member or not by its FP32
+ * distance unless that lies within band of (2h)^2, where the FP64 test of the
+ * stage-start positions decides (about one pair in 20 particles).  What is left
+ * in FP64 is the pair term of the members.  Members, terms and the order of the
+ * sums (the reference's list order) are those of the exact path's former kernel;
+ * the FMA path uses it as variant 8.
+ * A lane queues its members and sums them with its warp when a queue is nearly
+ * full, mostly once: queues of 64, emptied at 32, left 13.5 of 32 lanes active in
+ * the pair terms.  Bricks of 8 (3D) or 16 (2D) cells, 64 threads: small enough
+ * that a few thousand cells still fill the chip evenly.
+ * Exact path, shifting per step: 48x12x12 cells 13.1 -> 7.7 ms (73 % of the FP64
+ * pipe's issue slots in the SMs at work), 112x48 1.19 -> 0.58 ms; FMA path 200x200
+ * 1.48 -> 1.15 ms, 112x48 0.366 -> 0.332, 64x16x16 7.66 -> 7.64. */
+template <int D>
+struct SmallBrick;
+template <>
+struct SmallBrick<3> {
+  static constexpr int B0 = 2, B1 = 2, B2 = 2;
+};
+template <>
+struct SmallBrick<2> {
+  static constexpr int B0 = 4, B1 = 4, B2 = 1;
+};
+constexpr int PD_THREADS = 64, PD_BUF = 160;
+constexpr unsigned PD_CELL = 0x8000u; /* a queue's mark: the boundary particles of a staged cell */
+struct PdSmem {
+  int *off, *mid, *bnd; /* nsc + 1, nsc, nsc: entries, first appended entry, boundary flag of each staged cell */
+  float *blo, *bhi;     /* D nsc: bounds of its entries */
+  float4* ent;          /* cap */
+  unsigned short* buf;  /* PD_BUF x PD_THREADS queued members and marks */
+};
+__host__ __device__ inline size_t pd_layout(PdSmem* s, unsigned char* raw, int D, int nsc, int cap) {
+  size_t o = 0;
+  auto take = [&](size_t bytes) {
+    o = (o + 15) / 16 * 16;
+    const size_t r = o;
+    o += bytes;
+    return r;
+  };
+  const size_t ent = take(sizeof(float4) * (size_t)cap);
+  const size_t off = take(sizeof(int) * (size_t)(nsc + 1)), mid = take(sizeof(int) * (size_t)nsc);
+  const size_t bnd = take(sizeof(int) * (size_t)nsc);
+  const size_t blo = take(sizeof(float) * (size_t)(D * nsc)), bhi = take(sizeof(float) * (size_t)(D * nsc));
+  const size_t buf = take(sizeof(unsigned short) * PD_BUF * PD_THREADS);
+  if (s) {
+    s->ent = reinterpret_cast<float4*>(raw + ent);
+    s->off = reinterpret_cast<int*>(raw + off);
+    s->mid = reinterpret_cast<int*>(raw + mid);
+    s->bnd = reinterpret_cast<int*>(raw + bnd);
+    s->blo = reinterpret_cast<float*>(raw + blo);
+    s->bhi = reinterpret_cast<float*>(raw + bhi);
+    s->buf = reinterpret_cast<unsigned short*>(raw + buf);
+  }
+  return o;
+}
+
+template <int D, bool EX>
+__global__ void __launch_bounds__(PD_THREADS, 5) k_pst_d(CaseK K, DevPtrs<double> P, int xs, int hs, int xn, int hn, int nb0,
+                                                      int nb1, int cap) {
+  using BK = SmallBrick<D>;
+  extern __shared__ __align__(32) unsigned char smem_raw[];
+  const double dt = P.cnt->dt, max_v = P.cnt->max_v;
+  const double *XS = P.X[xs], *XN = P.X[xn], *HS = P.H[hs], *HN = P.H[hn];
+  const int b = blockIdx.x;
+  int c0[3];
+  c0[0] = (b / (nb0 * nb1)) * BK::B0;
+  c0[1] = ((b / nb0) % nb1) * BK::B1;
+  c0[2] = (D == 3) ? (b % nb0) * BK::B2 : 0;
+  const int bdim[3] = {BK::B0, BK::B1, D == 3 ? BK::B2 : 1};
+  int slo[3], sn[3];
+  double org[3];
+  float r2 = 0.f; /* the staged box's half diagonal, squared */
+  for (int d = 0; d < 3; d++) {
+    const int r = (d < D) ? K.rad2 : 0, Nd = (d < D) ? K.N[d] : 1;
+    slo[d] = max(c0[d] - r, 0);
+    sn[d] = min(c0[d] + bdim[d] - 1 + r, Nd - 1) - slo[d] + 1;
+    org[d] = (d < D) ? K.bl[d] + K.ps[d] * (c0[d] + 0.5 * bdim[d]) : 0.0;
+    const float e = (d < D) ? (float)K.ps[d] * (0.5f * (float)bdim[d] + (float)r) : 0.f;
+    r2 = fmaf(e, e, r2);
+  }
+  const int nsc = sn[0] * sn[1] * sn[2];
+  PdSmem sm;
+  pd_layout(&sm, smem_raw, D, nsc, cap);
+  __shared__ int s_red[SCAN_RED];
+  auto cell_of = [&](int l) {
+    const int t = l / (sn[1] * sn[2]), s = (l / sn[2]) % sn[1], m = l % sn[2];
+    return ((int64_t)(slo[0] + t) * K.N[1] + (slo[1] + s)) * K.N[2] + (slo[2] + m);
+  };
+  for (int l = threadIdx.x; l < nsc; l += blockDim.x) {
+    const int64_t c = cell_of(l);
+    const int cnt = min(P.bcnt[c], K.maxpc);
+    sm.off[l + 1] = cnt;
+    sm.mid[l] = cnt;
+    sm.bnd[l] = P.boff[c + 1] > P.boff[c] ? 1 : 0;
+  }
+  __syncthreads();
+  const bool use_sm = block_scan_counts(sm.off, nsc, s_red) <= cap;
+  if (use_sm) {
+    /* a warp takes several cells at a time, a quarter of it a cell */
+    const int q8 = threadIdx.x >> 3, l8 = threadIdx.x & 7;
+    for (int l = q8; l < nsc; l += PD_THREADS / 8) {
+      const int64_t c = cell_of(l);
+      const int e0 = sm.off[l], cnt = sm.off[l + 1] - e0;
+      float mn[3] = {1e30f, 1e30f, 1e30f}, mx[3] = {-1e30f, -1e30f, -1e30f};
+      int first = cnt;
+      for (int r = l8; r < cnt; r += 8) {
+        const int32_t q = P.bucket[c * K.maxpc + r];
+        if (P.lkey[q] >= KEY_APPEND && r < first) first = r;
+        float x[3] = {0.f, 0.f, 0.f};
+        for (int d = 0; d < D; d++) {
+          x[d] = (float)(XS[d * K.cap + q] - org[d]);
+          mn[d] = fminf(mn[d], x[d]);
+          mx[d] = fmaxf(mx[d], x[d]);
+          if (!(fabsf(x[d]) < 1e30f)) mn[d] = -1e30f, mx[d] = 1e30f; /* not a number: never pruned */
+        }
+        sm.ent[e0 + r] = make_float4(x[0], x[1], x[2], __int_as_float(q));
+      }
+      const unsigned g8 = 0xffu << (threadIdx.x & 24);
+      for (int o = 4; o > 0; o >>= 1) {
+        first = min(first, __shfl_xor_sync(g8, first, o));
+        for (int d = 0; d < D; d++) {
+          mn[d] = fminf(mn[d], __shfl_xor_sync(g8, mn[d], o));
+          mx[d] = fmaxf(mx[d], __shfl_xor_sync(g8, mx[d], o));
+        }
+      }
+      if (l8 == 0) {
+        sm.mid[l] = first;
+        for (int d = 0; d < D; d++) {
+          sm.blo[d * nsc + l] = mn[d];
+          sm.bhi[d * nsc + l] = mx[d];
+        }
+      }
+    }
+  }
+  /* the brick's own particles */
+  constexpr int nbc = BK::B0 * BK::B1 * BK::B2;
+  __shared__ int s_boff[nbc + 1];
+  __shared__ int s_bcell[nbc];
+  for (int q = threadIdx.x; q < nbc; q += blockDim.x) {
+    const int ci = c0[0] + q / (bdim[1] * bdim[2]), cj = c0[1] + (q / bdim[2]) % bdim[1], ck = c0[2] + q % bdim[2];
+    int cnt = 0;
+    int64_t c = -1;
+    if (ci < K.N[0] && cj < K.N[1] && ck < K.N[2]) {
+      c = ((int64_t)ci * K.N[1] + cj) * K.N[2] + ck;
+      cnt = min(P.bcnt[c], K.maxpc);
+    }
+    s_bcell[q] = (int)c;
+    s_boff[q + 1] = cnt;
+  }
+  __syncthreads();
+  const int npart = block_scan_counts(s_boff, nbc, s_red);
+  /* absolute error of an FP32 squared distance between staged positions, with room */
+  const float band = 4e-6f * r2;
+  for (int i = threadIdx.x; i < npart; i += blockDim.x) {
+    int q = 0, qh = nbc - 1;
+    while (q < qh) {
+      const int md = (q + qh + 1) >> 1;
+      if (s_boff[md] <= i) q = md;
+      else qh = md - 1;
+    }
+    const int64_t ci = s_bcell[q];
+    const int32_t p = P.bucket[ci * K.maxpc + (i - s_boff[q])];
+    PstPart<D, double, EX> pp;
+    pp.ph = P.phase[p];
+    for (int d = 0; d < 3; d++) pp.xsp[d] = pp.xnp[d] = 0.0;
+    for (int d = 0; d < D; d++) {
+      pp.xsp[d] = XS[d * K.cap + p];
+      pp.xnp[d] = XN[d * K.cap + p];
+    }
+    pp.hs_p = HS[p];
+    pp.hh = HN[p];
+    pp.rho_p = P.rho[p];
+    pp.c_p = P.c[p];
+    pp.init(K, max_v);
+    int pos[3], lo[3], hi[3];
+    cell_pos<D, double>(K, pp.xsp, pos);
+    bool inside = use_sm;
+    float xr[3] = {0.f, 0.f, 0.f};
+    for (int d = 0; d < 3; d++) {
+      const int r = (d < D) ? K.rad2 : 0;
+      lo[d] = max(pos[d] - r, 0);
+      hi[d] = min(pos[d] + r, (d < D ? K.N[d] : 1) - 1);
+      if (lo[d] < slo[d] || hi[d] >= slo[d] + sn[d]) inside = false;
+      if (d < D) xr[d] = (float)(pp.xsp[d] - org[d]);
+    }
+    if (!inside) {
+      pst_particle<D, double, EX, 0>(K, P, p, XS, XN, HS, HN, dt, max_v, nullptr);
+      continue;
+    }
+    const float lim = (float)pp.lim2, sure = lim * (1.f - 1e-6f) - band, never = lim * (1.f + 1e-6f) + band;
+    int nbuf = 0;
+    /* sum what is queued, in scan order, the next record in flight */
+    auto flush = [&]() {
+      unsigned v = PD_CELL;
+      int32_t q = 0;
+      double4 a = {};
+      auto fetch = [&](int k, unsigned& vv, int32_t& qq, double4& aa) {
+        vv = k < nbuf ? sm.buf[k * PD_THREADS + threadIdx.x] : PD_CELL;
+        if (!(vv & PD_CELL)) {
+          qq = __float_as_int(sm.ent[vv].w);
+          aa = reinterpret_cast<const double4*>(P.rec)[qq];
+        }
+      };
+      fetch(0, v, q, a);
+      for (int k = 0; k < nbuf; k++) {
+        unsigned vn;
+        int32_t qn = 0;
+        double4 an = {};
+        fetch(k + 1, vn, qn, an);
+        if (v & PD_CELL) pst_boundary_cell<D, double, EX>(K, P, cell_of((int)(v & (PD_CELL - 1))), pp);
+        else pst_rec_add<D, double, EX>(P, q, a, pp);
+        v = vn;
+        q = qn;
+        a = an;
+      }
+      nbuf = 0;
+    };
+    auto push = [&](unsigned v) {
+      if (nbuf == PD_BUF) flush();
+      sm.buf[nbuf++ * PD_THREADS + threadIdx.x] = (unsigned short)v;
+    };
+    auto queue = [&](int e) {
+      const float4 v = sm.ent[e];
+      const float dx = xr[0] - v.x, dy = xr[1] - v.y, dz = (D == 3) ? xr[2] - v.z : 0.f;
+      const float dd = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+      bool in = dd < sure;
+      if (!in && !(dd > never)) { /* also what is not a number */
+        const int32_t s = __float_as_int(v.w);
+        double xq[3] = {0, 0, 0};
+        for (int d = 0; d < D; d++) xq[d] = XS[d * K.cap + s];
+        in = pp.member(xq);
+      }
+      if (in) push((unsigned)e);
+    };
+    for (int t = lo[0]; t <= hi[0]; t++)
+      for (int s = lo[1]; s <= hi[1]; s++) {
+        int l = ((t - slo[0]) * sn[1] + (s - slo[1])) * sn[2] + (lo[2] - slo[2]);
+        for (int m = lo[2]; m <= hi[2]; m++, l++) {
+          const int e0 = sm.off[l], e1 = sm.off[l + 1], em = e0 + sm.mid[l];
+          float md = 0.f;
+          for (int d = 0; d < D; d++) {
+            const float g = fmaxf(fmaxf(sm.blo[d * nsc + l] - xr[d], xr[d] - sm.bhi[d * nsc + l]), 0.f);
+            md = fmaf(g, g, md);
+          }
+          const bool near = !(md * (1.f - 1e-6f) > never);
+          if (near)
+            for (int e = e0; e < em; e++) queue(e);
+          if (sm.bnd[l]) push(PD_CELL | (unsigned)l);
+          if (near)
+            for (int e = em; e < e1; e++) queue(e);
+          if (__any_sync(__activemask(), nbuf >= PD_BUF - 16)) flush();
+        }
+      }
+    flush();
+    pst_finish<D, double, EX>(K, P, p, dt, pp);
+  }
+}
+
+template <int D, bool EX>
+static void pst_d_launch(const CaseK& K, const DevPtrs<double>& P, int xs, int hs, int xn, int hn, cudaStream_t st) {
+  using BK = SmallBrick<D>;
+  const int nb0 = (D == 3) ? (K.N[2] + BK::B2 - 1) / BK::B2 : 1;
+  const int nb1 = (K.N[1] + BK::B1 - 1) / BK::B1;
+  const int nbx = (K.N[0] + BK::B0 - 1) / BK::B0;
+  const int r = K.rad2;
+  const int nsc = (BK::B0 + 2 * r) * (BK::B1 + 2 * r) * (D == 3 ? BK::B2 + 2 * r : 1);
+  /* staging room: half over the nominal count */
+  int cap = nsc * (D == 3 ? 8 : 4) * 3 / 2;
+  while ((pd_layout(nullptr, nullptr, D, nsc, cap) > 220 * 1024 || cap >= (int)PD_CELL) && cap > 256) cap = cap * 7 / 8;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaFuncSetAttribute(k_pst_d<D, EX>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+    attr_set = true;
+  }
+  k_pst_d<D, EX><<<nbx * nb1 * nb0, PD_THREADS, pd_layout(nullptr, nullptr, D, nsc, cap), st>>>(K, P, xs, hs, xn, hn, nb0, nb1,
+                                                                                               cap);
+}
+
 /* variants of the shifting kernel (the same members; results equal to rounding,
  * since variant 1 sums boundary particles in a second pass; the context's
  * autotuner times them on its own state and keeps the fastest): 0 per-lane row scan with
@@ -1735,10 +1920,10 @@ static void pst2_launch(const CaseK& K, const DevPtrs<R>& P, int xs, int hs, int
  * the cells with 512 threads, 5 over bricks of four times the cells with 1024
  * threads, 6 and 7 the second form (row-ordered records, global-row scan of
  * over-full bricks, packed pair arithmetic; 7 stages the records too).  The
- * exact path has one. */
+ * exact path has one; 8, on the FP64_FMA path, is that kernel (k_pst_d). */
 template <int D, typename R, bool EX>
 int Launch<D, R, EX>::pst_variants() {
-  return EX ? 1 : 8;
+  return EX ? 1 : sizeof(R) == 8 ? 9 : 8; /* 8: k_pst_d on the FMA path */
 }
 
 /* device scratch of the per-stage row sort (0 on the exact path) */
@@ -1773,19 +1958,21 @@ template <int D, typename R, bool EX>
 void Launch<D, R, EX>::pst(const CaseK& K, const DevPtrs<R>& P, int xs, int hs, int xn, int hn, int var,
                            void* scratch, cudaStream_t st) {
   if constexpr (EX) {
-    pst_launch<D, R, EX, 0>(K, P, xs, hs, xn, hn, RowSorted<R>{}, st);
+    pst_d_launch<D, EX>(K, P, xs, hs, xn, hn, st);
   } else {
     RowSortBufs<R> B;
     rowsort_layout<R>(K, static_cast<unsigned char*>(scratch), &B);
     const RowSorted<R> RS{B.row, B.rec, B.rk, B.pmin, B.pmax};
-    if (var == 1) pst_launch<D, R, EX, 1>(K, P, xs, hs, xn, hn, RS, st);
-    else if (var == 2) pst_launch<D, R, EX, 2>(K, P, xs, hs, xn, hn, RS, st);
-    else if (var == 3) pst_launch<D, R, EX, 3>(K, P, xs, hs, xn, hn, RS, st);
-    else if (var == 4) pst_launch<D, R, EX, 5>(K, P, xs, hs, xn, hn, RS, st);
-    else if (var == 5) pst_launch<D, R, EX, 6>(K, P, xs, hs, xn, hn, RS, st);
+    if constexpr (sizeof(R) == 8)
+      if (var == 8) return pst_d_launch<D, EX>(K, P, xs, hs, xn, hn, st);
+    if (var == 1) pst_launch<D, R, 1>(K, P, xs, hs, xn, hn, RS, st);
+    else if (var == 2) pst_launch<D, R, 2>(K, P, xs, hs, xn, hn, RS, st);
+    else if (var == 3) pst_launch<D, R, 3>(K, P, xs, hs, xn, hn, RS, st);
+    else if (var == 4) pst_launch<D, R, 5>(K, P, xs, hs, xn, hn, RS, st);
+    else if (var == 5) pst_launch<D, R, 6>(K, P, xs, hs, xn, hn, RS, st);
     else if (var == 6) pst2_launch<D, R, false>(K, P, xs, hs, xn, hn, RS, st);
     else if (var == 7) pst2_launch<D, R, true>(K, P, xs, hs, xn, hn, RS, st);
-    else pst_launch<D, R, EX, 0>(K, P, xs, hs, xn, hn, RS, st);
+    else pst_launch<D, R, 0>(K, P, xs, hs, xn, hn, RS, st);
   }
 }
 

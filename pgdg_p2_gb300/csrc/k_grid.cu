@@ -16,6 +16,11 @@ constexpr int BLK = 256;
 #define GRID_STRIDE(i, n) for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); \
                                i += (int64_t)gridDim.x * blockDim.x)
 
+/* threads per block of the per-cell kernels: blocks of 32 or 64 spread a grid of a
+ * few thousand cells, whose time is the latency of one cell's chain, over all SMs
+ * (blocks of 128 filled 42 of 152 at 112x48 cells) */
+inline int spread(int64_t n) { return n <= 152 * 8 * 32 ? 32 : n <= 152 * 8 * 64 ? 64 : 128; }
+
 template <int D>
 __device__ __forceinline__ void cijk(const CaseK& K, int64_t ci, int* idx) {
   idx[2] = (int)(ci % K.N[2]);
@@ -449,7 +454,7 @@ void Launch<D, R, EX>::p2g(const CaseK& K, const DevPtrs<R>& P, bool fresh_bins,
   const double hi = K.p_g * 1 * 3.2 / CUT_OFF;
   double hh = (D == 2) ? hi * hi : hi * hi * hi;
   double Cw = (D == 2) ? 1.0 / PI_REF / hh * 7. / 4. : 1.0 / PI_REF / hh * 21. / 16.;
-  k_p2g<D, R, EX><<<grid_for(K.ncell, 128), 128, 0, st>>>(K, P, Cw, fresh_bins ? p2g_skip<D>(K) : 0);
+  k_p2g<D, R, EX><<<grid_for(K.ncell, spread(K.ncell)), spread(K.ncell), 0, st>>>(K, P, Cw, fresh_bins ? p2g_skip<D>(K) : 0);
 }
 
 /* the newly present phases k_p2g flagged (runs after it) */
@@ -458,7 +463,7 @@ void Launch<D, R, EX>::p2g_new(const CaseK& K, const DevPtrs<R>& P, cudaStream_t
   const double hi = K.p_g * 1 * 3.2 / CUT_OFF;
   double hh = (D == 2) ? hi * hi : hi * hi * hi;
   double Cw = (D == 2) ? 1.0 / PI_REF / hh * 7. / 4. : 1.0 / PI_REF / hh * 21. / 16.;
-  k_p2g_new<D, R, EX><<<grid_for(K.ncell, 128), 128, 0, st>>>(K, P, Cw);
+  k_p2g_new<D, R, EX><<<grid_for(K.ncell, spread(K.ncell)), spread(K.ncell), 0, st>>>(K, P, Cw);
 }
 
 /* ------------------------------------------------------------------ */
@@ -675,7 +680,7 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(6)) k_limiter(CaseK K, D
 
 template <int D, typename R, bool EX>
 void Launch<D, R, EX>::limiter(const CaseK& K, const DevPtrs<R>& P, cudaStream_t st) {
-  k_limiter<D, R, EX><<<grid_for(K.ncell, 128), 128, 0, st>>>(K, P);
+  k_limiter<D, R, EX><<<grid_for(K.ncell, spread(K.ncell)), spread(K.ncell), 0, st>>>(K, P);
 }
 
 /* ------------------------------------------------------------------ */
@@ -713,6 +718,28 @@ __device__ __forceinline__ void flux_col(const R* Uu, const R* v, R Pp, int a, R
   if (esh != R(0)) Fc[U - 1] += va * esh;   /* (E_true + p) v with E_true = E + esh */
 }
 
+/* lanes per cell of the residual: on the FP64 paths a lane takes one face (and one
+ * the volume integral), since one cell is a chain of 16,000 dependent FP64
+ * instructions (48x12x12 cells: 1.51 ms per launch with a thread per cell, 0.60
+ * with eight); the lanes' parts are added in the order of the serial loop */
+template <typename R>
+__host__ __device__ constexpr int acc_lanes() {
+  return sizeof(R) == 8 ? 8 : 1;
+}
+/* interface problems of cell idx's phase ss on face f */
+template <int D, typename R>
+__device__ __forceinline__ int face_problems(const CaseK& K, const int* idx, int f, int ss, const R* calph) {
+  const int a = (f == 0 || f == 2) ? 1 : (f == 1 || f == 3) ? 0 : 2;
+  int nb[3] = {idx[0], idx[1], idx[2]};
+  nb[a] += (f == 0 || f == 3 || f == 4) ? -1 : 1;
+  if (nb[a] < 0 || nb[a] >= K.N[a]) return 0;
+  const int64_t cn = cidx3(K, nb[0], nb[1], nb[2]);
+  int n = 0;
+  for (int s1 = 0; s1 < F; s1++)
+    if (s1 != ss && calph[s1 * K.ncell + cn] != R(0)) n += (D == 3) ? 4 : 2;
+  return n;
+}
+
 /* MODE 0: MGFM solved inline; MODE 2: queue every interface problem (no flux
  * work); MODE 3: read the ghost states of the interface problems from the queue */
 template <int D, typename R, bool EX, int MODE>
@@ -734,7 +761,13 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
     const bool over = Q.tot[0] > (unsigned long long)Q.cap;
     if ((MODE == 3 && over) || (MODE == 0 && !over)) return;
   }
-  GRID_STRIDE(ci, nc) {
+  constexpr int G = acc_lanes<R>();
+  const int sub = (int)threadIdx.x & (G - 1);
+  const unsigned gmask = G == 1 ? 0u : 0xffu << (threadIdx.x & 24);
+  __shared__ R s_part[G == 1 ? 1 : 128 / G][G == 1 ? 1 : NF + 1][G == 1 ? 1 : U * B];
+  auto* part = s_part[G == 1 ? 0 : threadIdx.x / G];
+  for (int64_t ci = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / G; ci < nc;
+       ci += (int64_t)gridDim.x * blockDim.x / G) {
     if (!P.cused[ci]) continue;
     int idx[3];
     cijk<D>(K, ci, idx);
@@ -742,15 +775,27 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
     if constexpr (EX) center<D>(K, idx, xc);
     const bool mirror_j = (idx[1] == K.N[1] - 1 || idx[1] == 0);
     const bool mirror_k = (D == 3) && (idx[2] == K.N[2] - 1 || idx[2] == 0);
-    int64_t qi = 0;
+    int64_t qi = 0, qcell = 0;
     if constexpr (MODE != 0) {
       if (Q.off[ci + 1] == Q.off[ci]) {
         if constexpr (MODE == 2) continue;
       }
-      qi = (int64_t)Q.off[ci];
+      qcell = qi = (int64_t)Q.off[ci];
     }
     for (int ss = 0; ss < F; ss++) {
       if (P.cph[ss * nc + ci] != 1) continue;
+      if constexpr (G > 1 && MODE != 0) {
+        /* a lane's problems follow those of the faces before its own */
+        const int mine = sub < NF ? face_problems<D, R>(K, idx, sub, ss, P.calph) : 0;
+        int inc = mine;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+          const int y = __shfl_up_sync(gmask, inc, o, G);
+          if (sub >= o) inc += y;
+        }
+        qi = qcell + inc - mine;
+        qcell += __shfl_sync(gmask, inc, G - 1, G);
+      }
       const R gs = (R)K.gamma[ss], pfs = (R)K.pinf[ss], pfe = (R)K.pinf_eos[ss], esh = (R)K.eshift[ss];
       R co[U][B], L[U], dc[U][B];
       for (int u = 0; u < U; u++) {
@@ -762,7 +807,7 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
       }
       /* volume integral, 2^D Gauss points */
       const R voli = (R)voli_d;
-      for (int g = 0; g < (MODE == 2 ? 0 : NG); g++) {
+      for (int g = 0; g < (MODE == 2 || (G > 1 && sub != NF) ? 0 : NG); g++) {
         int g1 = (D == 3) ? (g >> 2) : (g >> 1), g2 = (D == 3) ? ((g >> 1) & 1) : (g & 1), g3 = g & 1;
         R dp[3];
         if constexpr (EX) {
@@ -793,7 +838,7 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
         }
       }
       /* face integral */
-      for (int f = 0; f < NF; f++) {
+      for (int f = G > 1 ? sub : 0; f < (G > 1 ? min(sub + 1, NF) : NF); f++) {
         /* exact path: the reference's absolute FP64 face geometry; otherwise
          * the same face relative to the cell centre in R */
         FaceK fc;
@@ -1041,9 +1086,25 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
         }
         const R Sj = EX ? (R)fc.S : fr.S;
         for (int b = 0; b < B; b++)
-          for (int u = 0; u < U; u++) dc[u][b] += (-DFn[b][u] * na) * Sj;
+          for (int u = 0; u < U; u++) {
+            if constexpr (G > 1) dc[u][b] = (-DFn[b][u] * na) * Sj;
+            else dc[u][b] += (-DFn[b][u] * na) * Sj;
+          }
       }
       if constexpr (MODE == 2) continue;
+      if constexpr (G > 1) {
+        if (sub <= NF)
+          for (int u = 0; u < U; u++)
+            for (int b = 0; b < B; b++) part[sub][u * B + b] = dc[u][b];
+        __syncwarp(gmask);
+        for (int t = sub; t < U * B; t += G) {
+          R acc = part[NF][t];
+          for (int f = 0; f < NF; f++) acc += part[f][t];
+          P.cdcoef[(ss * U * B + t) * nc + ci] = acc * (t % B == 0 ? inv[0] : t % B == 1 ? inv[1] : t % B == 2 ? inv[2] : inv[3]);
+        }
+        __syncwarp(gmask);
+        continue;
+      }
       for (int u = 0; u < U; u++)
         for (int b = 0; b < B; b++) P.cdcoef[((ss * U + u) * B + b) * nc + ci] = dc[u][b] * inv[b];
     }
@@ -1094,12 +1155,13 @@ __global__ void k_iface_total(const unsigned long long* blk, int nblk, unsigned 
 
 template <int D, typename R, bool EX>
 void Launch<D, R, EX>::grid_acc(const CaseK& K, const DevPtrs<R>& P, cudaStream_t st) {
+  const int64_t nth = acc_lanes<R>() * K.ncell;
   double voli = K.ps[0] * K.ps[1];
   if (D == 3) voli = voli * K.ps[2];
   double ps[3] = {K.ps[0] / 2, K.ps[1] / 2, K.ps[2] / 2};
   double m1 = (ps[0] * ps[0] / 3.) * voli, m2 = (ps[1] * ps[1] / 3.) * voli, m3 = (ps[2] * ps[2] / 3.) * voli;
   IfaceQ Q{};
-  k_grid_acc<D, R, EX, 0><<<grid_for(K.ncell, 128), 128, 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
+  k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
 }
 
 /* count, offsets and gather of the stage's interface problems, all on the
@@ -1107,24 +1169,26 @@ void Launch<D, R, EX>::grid_acc(const CaseK& K, const DevPtrs<R>& P, cudaStream_
  * queue holds batches none of them and the residual solves it inline */
 template <int D, typename R, bool EX>
 void Launch<D, R, EX>::iface_gather(const CaseK& K, const DevPtrs<R>& P, IfaceQ Q, cudaStream_t st) {
+  const int64_t nth = acc_lanes<R>() * K.ncell;
   double voli = K.ps[0] * K.ps[1];
   if (D == 3) voli = voli * K.ps[2];
   k_iface_count<D, R, EX><<<grid_for(K.ncell, BLK), BLK, 0, st>>>(K, P, Q.off);
   scan_u64(Q.off, Q.blk, Q.d_ncell, K.ncell, st);
   const int nblk = (int)((K.ncell + 2047) / 2048);
   k_iface_total<R, EX><<<1, 1, 0, st>>>(Q.blk, nblk, Q.off, K.ncell, Q.tot, Q.cap);
-  k_grid_acc<D, R, EX, 2><<<grid_for(K.ncell, 128), 128, 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
+  k_grid_acc<D, R, EX, 2><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
 }
 
 template <int D, typename R, bool EX>
 void Launch<D, R, EX>::grid_acc_queued(const CaseK& K, const DevPtrs<R>& P, IfaceQ Q, cudaStream_t st) {
+  const int64_t nth = acc_lanes<R>() * K.ncell;
   double voli = K.ps[0] * K.ps[1];
   if (D == 3) voli = voli * K.ps[2];
   double ps[3] = {K.ps[0] / 2, K.ps[1] / 2, K.ps[2] / 2};
   double m1 = (ps[0] * ps[0] / 3.) * voli, m2 = (ps[1] * ps[1] / 3.) * voli, m3 = (ps[2] * ps[2] / 3.) * voli;
-  k_grid_acc<D, R, EX, 3><<<grid_for(K.ncell, 128), 128, 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
+  k_grid_acc<D, R, EX, 3><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
   /* the inline solve of a stage that outgrew the queue (returns at once otherwise) */
-  k_grid_acc<D, R, EX, 0><<<grid_for(K.ncell, 128), 128, 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
+  k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
 }
 
 /* ------------------------------------------------------------------ */
@@ -1221,7 +1285,7 @@ __global__ void __launch_bounds__(256) k_update_grid(CaseK K, DevPtrs<R> P, int 
 
 template <int D, typename R, bool EX>
 void Launch<D, R, EX>::update_grid(const CaseK& K, const DevPtrs<R>& P, int md, cudaStream_t st) {
-  k_update_grid<D, R, EX><<<grid_for(K.ncell, BLK), BLK, 0, st>>>(K, P, md);
+  k_update_grid<D, R, EX><<<grid_for(K.ncell, spread(K.ncell)), spread(K.ncell), 0, st>>>(K, P, md);
 }
 
 /* ------------------------------------------------------------------ */

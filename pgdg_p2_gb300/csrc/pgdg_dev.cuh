@@ -230,7 +230,7 @@ struct Launch {
   static void p2g_new(const CaseK&, const DevPtrs<R>&, cudaStream_t);
   static void limiter(const CaseK&, const DevPtrs<R>&, cudaStream_t);
   static void grid_acc(const CaseK&, const DevPtrs<R>&, cudaStream_t);
-  /* queued variant: returns the number of interface problems (negative: over capacity) */
+  /* the stage's interface problems queued, and the residual with their ghost states */
   static void iface_gather(const CaseK&, const DevPtrs<R>&, IfaceQ, cudaStream_t);
   static void grid_acc_queued(const CaseK&, const DevPtrs<R>&, IfaceQ, cudaStream_t);
   static void update_grid(const CaseK&, const DevPtrs<R>&, int md, cudaStream_t);

@@ -967,7 +967,7 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
                   gh[1] = Q.out3[3 * e + 1];
                   gh[2] = Q.out3[3 * e + 2];
                 } else {
-                  int it = mgfm<false>((double)vni, (double)vnj, (double)P_i, (double)P_j, (double)rho_i, (double)rho_j,
+                  int it = mgfm_serial((double)vni, (double)vnj, (double)P_i, (double)P_j, (double)rho_i, (double)rho_j,
                                 K.gamma[ss], K.pinf[ss], K.gamma[s1], K.pinf[s1], variant, -1.0, gh);
                   ncall++;
                   nit += it;

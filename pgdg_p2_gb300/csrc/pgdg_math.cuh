@@ -177,10 +177,7 @@ PGDG_HD double jaco_cal(double W, double y, double d, double rhol, double g) {
  * tolerance no iterate on the way converges.  The iterates down to 4e-8 are then
  * p - 0.6 p, two operations in place of about 130, and the rest runs as usual: the
  * same bits and counts.  descent = 1 looks for this at once (the caller knows
- * that f(1e-8) < 0), 0 after two capped steps downwards; DESCENT = false leaves it
- * out (the residual's inline solves converge in two or three iterations, and the
- * registers count there). */
-template <bool DESCENT = true>
+ * that f(1e-8) < 0), 0 after two capped steps downwards. */
 PGDG_HD int mgfm(double ul, double ur, double pl, double pr, double rhol, double rhor, double gl,
                  double pinfl, double gr, double pinfr, int variant, double seed_p, double out[3], int descent = 0) {
   double pstar;
@@ -201,7 +198,7 @@ PGDG_HD int mgfm(double ul, double ur, double pl, double pr, double rhol, double
   double f1 = 1., Wl = 0, ql = 0, pold = pstar, usl;
   int nn = 0, down = descent ? 2 : 0;
   do {
-    if (DESCENT && down == 2) {
+    if (down == 2) {
       down = 3; /* looked at once */
       /* the convexity above holds for these; the margins cover the rounding of f */
       if (pstar > 4e-8 && pstar < 1e100 && rhol > 0 && rhor > 0 && gl > 1 && gr > 1 && pinfl >= 0 && pinfr >= 0) {
@@ -243,6 +240,68 @@ PGDG_HD int mgfm(double ul, double ur, double pl, double pr, double rhol, double
   if (variant == 0) usl = dsub(ul, ql);
   else usl = dsub(ul, ddiv(dsub(pstar, pl), Wl));
   out[0] = rhols_cal(rhol, pl, pold, gl, pinfl);
+  out[1] = pstar;
+  out[2] = usl;
+  return nn;
+}
+
+/* The same solve without the shared reciprocals and the replay, for the FP32
+ * residual's inline calls (two or three iterations each, where neither pays
+ * much): inlined there, any other form of it changes how the compiler contracts
+ * the FP32 arithmetic around the call, and with it the residual's rounding. */
+PGDG_HD double jaco_serial(double W, double pl, double rhol, double ps, double g) {
+  double t = ddiv(dsub(ps, pl), dmul(W, W));
+  t = dmul(t, rhol);
+  t = dmul(t, dadd(g, 1));
+  t = ddiv(t, 4.);
+  t = ddiv(t, W);
+  return dsub(ddiv(1., W), t);
+}
+
+PGDG_HD int mgfm_serial(double ul, double ur, double pl, double pr, double rhol, double rhor, double gl,
+                 double pinfl, double gr, double pinfr, int variant, double seed_p, double out[3]) {
+  double pstar;
+  if (variant == 0) {
+    pl = amax1(pl, 1e-10);
+    pr = amax1(pr, 1e-10);
+    rhol = amax1(rhol, 1e-10);
+    rhor = amax1(rhor, 1e-10);
+    pstar = amax1(pl, pr);
+  } else {
+    if (pl < 0) pl = 0;
+    if (pr < 0) pr = 0;
+    pstar = dmul(dadd(pl, pr), 0.5);
+  }
+  if (seed_p > 0) pstar = seed_p;
+  double tol = amax1(1e-8, dmul(1e-3, fabs(dsub(ul, ur))));
+  double f1 = 1.;
+  double rhols = 0, usl = 0, Wl = 0, Wr = 0;
+  int nn = 0;
+  do {
+    Wl = wl_cal(rhol, pl, pstar, gl, pinfl);
+    Wr = wl_cal(rhor, pr, pstar, gr, pinfr);
+    if (variant == 0) usl = dsub(ul, ddiv(dsub(pstar, pl), Wl));
+    rhols = rhols_cal(rhol, pl, pstar, gl, pinfl);
+    f1 = dsub(dsub(dsub(ul, ur), ddiv(dsub(pstar, pl), Wl)), ddiv(dsub(pstar, pr), Wr));
+    double jac = dsub(-jaco_serial(Wl, pl, rhol, pstar, gl), jaco_serial(Wr, pr, rhor, pstar, gr));
+    double dp = ddiv(-f1, jac);
+    double cap = dmul(0.6, pstar);
+    if (fabs(dp) > cap) dp = copysign(cap, dp);
+    const double pold = pstar;
+    pstar = dadd(pstar, dp);
+    pstar = amax1(pstar, 1e-8);
+    nn++;
+    /* every quantity of an iteration is a function of pstar alone: once an
+     * unconverged iterate repeats (the 1e-8 floor of a problem without a
+     * positive root) the remaining iterations up to the cap reproduce it bit
+     * for bit, so leave with the cap count the full loop would report */
+    if (pstar == pold && fabs(f1) > tol) {
+      nn = 50;
+      break;
+    }
+  } while (fabs(f1) > tol && nn < 50);
+  if (variant != 0) usl = dsub(ul, ddiv(dsub(pstar, pl), Wl));
+  out[0] = rhols;
   out[1] = pstar;
   out[2] = usl;
   return nn;

@@ -154,6 +154,7 @@ struct Ctx : pgdg_ctx {
   int x0b = 0;          /* step-start coordinate buffer (md 1) */
   double* d_tot = nullptr;
   IfaceQ Q{};
+  int64_t q_room = 0; /* problems the queue's buffers hold (Q.cap: those a queued stage may use) */
   PartScratch part;   /* root partition of the interface batch */
   unsigned char* pst_scratch = nullptr; /* per-stage row sort of the shifting kernel */
   /* every particle lies in its bucket's cell (true from binning until the
@@ -281,9 +282,10 @@ struct Ctx : pgdg_ctx {
      * sized for a few per cent of the cells, grown on demand when the queue was asked
      * for (a stage that outgrows it is solved inline) */
     Q.cap = std::max<int64_t>(1 << 16, sizeof(R) == 8 ? K.ncell : K.ncell / 8);
-    CK(A(&Q.in6, 6 * (size_t)Q.cap));
-    CK(A(&Q.mat, 2 * (size_t)Q.cap));
-    CK(A(&Q.out3, 3 * (size_t)Q.cap));
+    q_room = std::max<int64_t>(Q.cap, K.ncell / 2); /* of the mixed path without a surrogate */
+    CK(A(&Q.in6, 6 * (size_t)q_room));
+    CK(A(&Q.mat, 2 * (size_t)q_room));
+    CK(A(&Q.out3, 3 * (size_t)q_room));
     CK(A(&Q.off, nc + 1));
     CK(A(&Q.blk, (nc + 2047) / 2048 + 2));
     CK(A(&Q.tot, 2));
@@ -922,7 +924,7 @@ struct Ctx : pgdg_ctx {
         if (a == p) a = nullptr;
       cudaFree(p);
     }
-    Q.cap = need;
+    Q.cap = q_room = need;
     CK(A(&Q.in6, 6 * (size_t)Q.cap));
     CK(A(&Q.mat, 2 * (size_t)Q.cap));
     CK(A(&Q.out3, 3 * (size_t)Q.cap));
@@ -955,10 +957,24 @@ struct Ctx : pgdg_ctx {
     return PGDG_OK;
   }
   int grid_acc() override {
-    /* FP32 residual without the queue: solved inline, as its rounding differs
-     * between the inline and the queued build */
+    /* FP32 without a surrogate: the same batch, gathered and used by the inline
+     * residual's own code (its FP32 arithmetic is contracted otherwise in the queued
+     * builds).  Inline, a warp runs its cells' problems one after another at 64 cycles
+     * an FP64 instruction, however few of its lanes have one.  Per step: 112x48 cells
+     * 0.39 -> 0.20 ms, with three materials 0.74 -> 0.25, 171x45x39 cells 1.92 -> 0.96 */
     if (!iface_queue && sizeof(R) == 4) {
-      timed("grid_acc", 1, [&] { Launch<D, R, EX>::grid_acc(K, P, st); });
+      IfaceQ q = Q;
+      if (iface_cap_fixed < 0) q.cap = q_room;
+      q.phase = 1;
+      timed("iface_gather", 6, [&] { Launch<D, R, EX>::iface_gather(K, P, q, st); });
+      int rc = PGDG_OK;
+      timed("mgfm_seeded", 1, [&] {
+        rc = mgfm_seeded_run(nullptr, q.in6, q.mat, d_gam, d_pinf, K.mgfm_variant, q.out3, nullptr, q.cap,
+                             &P.cnt->mgfm_calls, part, st, q.tot + 1);
+      });
+      if (rc) return rc;
+      q.phase = 2;
+      timed("grid_acc", 1, [&] { Launch<D, R, EX>::grid_acc(K, P, q, st); });
       return PGDG_OK;
     }
     /* queue the interface problems, solve them in one batch (from the surrogate's

@@ -740,7 +740,7 @@ __device__ __forceinline__ int face_problems(const CaseK& K, const int* idx, int
   return n;
 }
 
-/* MODE 0: MGFM solved inline; MODE 2: queue every interface problem (no flux
+/* MODE 0: MGFM solved inline (FP32: or gathered and used, see phase); MODE 2: queue every interface problem (no flux
  * work); MODE 3: read the ghost states of the interface problems from the queue */
 template <int D, typename R, bool EX, int MODE>
 __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_grid_acc(CaseK K, DevPtrs<R> P, int variant, double voli_d,
@@ -759,8 +759,13 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
    * solve (MODE 0 launched beside MODE 3): exactly one of the two does work */
   if (Q.tot) {
     const bool over = Q.tot[0] > (unsigned long long)Q.cap;
-    if ((MODE == 3 && over) || (MODE == 0 && !over)) return;
+    if ((MODE == 3 && over) || (MODE == 0 && !over && (sizeof(R) == 8 || Q.phase == 0))) return;
   }
+  /* FP32 without a surrogate: the same compiled code gathers the problems, and runs
+   * again with the batch's results (those beyond the queue solved here), so that
+   * problems and residual round as in the inline solve */
+  constexpr bool PH = MODE == 0 && sizeof(R) == 4;
+  const int phase = PH ? Q.phase : 0;
   constexpr int G = acc_lanes<R>();
   const int sub = (int)threadIdx.x & (G - 1);
   const unsigned gmask = G == 1 ? 0u : 0xffu << (threadIdx.x & 24);
@@ -781,6 +786,10 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
         if constexpr (MODE == 2) continue;
       }
       qcell = qi = (int64_t)Q.off[ci];
+    }
+    if (PH && phase != 0) {
+      if (phase == 1 && Q.off[ci + 1] == Q.off[ci]) continue;
+      qi = (int64_t)Q.off[ci];
     }
     for (int ss = 0; ss < F; ss++) {
       if (P.cph[ss * nc + ci] != 1) continue;
@@ -871,7 +880,7 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
           if (fbound == 0) {
             ajo = P.calph[so * nc + nb];
             if (ajo == R(0)) continue;
-            if (MODE == 2 && so == ss) continue;
+            if ((MODE == 2 || (PH && phase == 1)) && so == ss) continue;
             for (int u = 0; u < U; u++) {
               for (int b = 0; b < B; b++) cn[u][b] = P.ccoef[((so * U + u) * B + b) * nc + nb];
               ln[u] = P.clim[(so * U + u) * nc + nb];
@@ -967,11 +976,32 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
                   gh[1] = Q.out3[3 * e + 1];
                   gh[2] = Q.out3[3 * e + 2];
                 } else {
-                  int it = mgfm_serial((double)vni, (double)vnj, (double)P_i, (double)P_j, (double)rho_i, (double)rho_j,
-                                K.gamma[ss], K.pinf[ss], K.gamma[s1], K.pinf[s1], variant, -1.0, gh);
-                  ncall++;
-                  nit += it;
-                  if (it >= 50) nmax++;
+                  const int64_t e = PH && phase != 0 ? qi++ : Q.cap;
+                  if (PH && e < Q.cap) {
+                    double* q6 = Q.in6 + 6 * e;
+                    if (phase == 1) {
+                      q6[0] = (double)vni;
+                      q6[1] = (double)vnj;
+                      q6[2] = (double)P_i;
+                      q6[3] = (double)P_j;
+                      q6[4] = (double)rho_i;
+                      q6[5] = (double)rho_j;
+                      Q.mat[2 * e] = (int8_t)ss;
+                      Q.mat[2 * e + 1] = (int8_t)s1;
+                      continue;
+                    }
+                    gh[0] = Q.out3[3 * e];
+                    gh[1] = Q.out3[3 * e + 1];
+                    gh[2] = Q.out3[3 * e + 2];
+                  } else {
+                    if (PH && phase == 1) continue;
+                    int it = mgfm_serial((double)vni, (double)vnj, (double)P_i, (double)P_j, (double)rho_i,
+                                         (double)rho_j, K.gamma[ss], K.pinf[ss], K.gamma[s1], K.pinf[s1], variant,
+                                         -1.0, gh);
+                    ncall++;
+                    nit += it;
+                    if (it >= 50) nmax++;
+                  }
                 }
                 rho_j = (R)gh[0];
                 P_j = (R)gh[1];
@@ -1105,6 +1135,7 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
         __syncwarp(gmask);
         continue;
       }
+      if (PH && phase == 1) continue;
       for (int u = 0; u < U; u++)
         for (int b = 0; b < B; b++) P.cdcoef[((ss * U + u) * B + b) * nc + ci] = dc[u][b] * inv[b];
     }
@@ -1146,21 +1177,21 @@ __global__ void k_iface_count(CaseK K, DevPtrs<R> P, unsigned long long* cnt) {
 }
 template <typename R, bool EX>
 __global__ void k_iface_total(const unsigned long long* blk, int nblk, unsigned long long* off, int64_t nc,
-                              unsigned long long* tot, int64_t cap) {
+                              unsigned long long* tot, int64_t cap, int some) {
   const unsigned long long n = blk[nblk];
   off[nc] = n;
   tot[0] = n;
-  tot[1] = n <= (unsigned long long)cap ? n : 0ull; /* an overflowing stage batches nothing */
+  /* an overflowing stage batches nothing, or (some) what the queue holds */
+  tot[1] = n <= (unsigned long long)cap ? n : some ? (unsigned long long)cap : 0ull;
 }
 
 template <int D, typename R, bool EX>
-void Launch<D, R, EX>::grid_acc(const CaseK& K, const DevPtrs<R>& P, cudaStream_t st) {
+void Launch<D, R, EX>::grid_acc(const CaseK& K, const DevPtrs<R>& P, IfaceQ Q, cudaStream_t st) {
   const int64_t nth = acc_lanes<R>() * K.ncell;
   double voli = K.ps[0] * K.ps[1];
   if (D == 3) voli = voli * K.ps[2];
   double ps[3] = {K.ps[0] / 2, K.ps[1] / 2, K.ps[2] / 2};
   double m1 = (ps[0] * ps[0] / 3.) * voli, m2 = (ps[1] * ps[1] / 3.) * voli, m3 = (ps[2] * ps[2] / 3.) * voli;
-  IfaceQ Q{};
   k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
 }
 
@@ -1175,8 +1206,9 @@ void Launch<D, R, EX>::iface_gather(const CaseK& K, const DevPtrs<R>& P, IfaceQ 
   k_iface_count<D, R, EX><<<grid_for(K.ncell, BLK), BLK, 0, st>>>(K, P, Q.off);
   scan_u64(Q.off, Q.blk, Q.d_ncell, K.ncell, st);
   const int nblk = (int)((K.ncell + 2047) / 2048);
-  k_iface_total<R, EX><<<1, 1, 0, st>>>(Q.blk, nblk, Q.off, K.ncell, Q.tot, Q.cap);
-  k_grid_acc<D, R, EX, 2><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
+  k_iface_total<R, EX><<<1, 1, 0, st>>>(Q.blk, nblk, Q.off, K.ncell, Q.tot, Q.cap, Q.phase);
+  if (Q.phase) k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
+  else k_grid_acc<D, R, EX, 2><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
 }
 
 template <int D, typename R, bool EX>
@@ -1485,7 +1517,7 @@ void Launch<D, R, EX>::probe(const CaseK& K, const DevPtrs<R>& P, double* d_scra
   template void Launch<D, R, EX>::p2g(const CaseK&, const DevPtrs<R>&, bool, cudaStream_t);        \
   template void Launch<D, R, EX>::p2g_new(const CaseK&, const DevPtrs<R>&, cudaStream_t);          \
   template void Launch<D, R, EX>::limiter(const CaseK&, const DevPtrs<R>&, cudaStream_t);          \
-  template void Launch<D, R, EX>::grid_acc(const CaseK&, const DevPtrs<R>&, cudaStream_t);         \
+  template void Launch<D, R, EX>::grid_acc(const CaseK&, const DevPtrs<R>&, IfaceQ, cudaStream_t);         \
   template void Launch<D, R, EX>::iface_gather(const CaseK&, const DevPtrs<R>&, IfaceQ, cudaStream_t); \
   template void Launch<D, R, EX>::grid_acc_queued(const CaseK&, const DevPtrs<R>&, IfaceQ, cudaStream_t); \
   template void Launch<D, R, EX>::update_grid(const CaseK&, const DevPtrs<R>&, int, cudaStream_t); \

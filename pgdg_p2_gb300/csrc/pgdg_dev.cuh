@@ -160,6 +160,7 @@ struct IfaceQ {
    * when [0] exceeds cap (the residual then solves the stage inline) */
   unsigned long long* tot;
   int64_t cap;
+  int phase; /* the mixed path's residual (MODE 0): 0 solve inline, 1 gather, 2 use the batch's results */
 };
 
 /* ---------------- cell ids ---------------- */
@@ -229,7 +230,7 @@ struct Launch {
   static void p2g(const CaseK&, const DevPtrs<R>&, bool fresh_bins, cudaStream_t);
   static void p2g_new(const CaseK&, const DevPtrs<R>&, cudaStream_t);
   static void limiter(const CaseK&, const DevPtrs<R>&, cudaStream_t);
-  static void grid_acc(const CaseK&, const DevPtrs<R>&, cudaStream_t);
+  static void grid_acc(const CaseK&, const DevPtrs<R>&, IfaceQ, cudaStream_t);
   /* the stage's interface problems queued, and the residual with their ghost states */
   static void iface_gather(const CaseK&, const DevPtrs<R>&, IfaceQ, cudaStream_t);
   static void grid_acc_queued(const CaseK&, const DevPtrs<R>&, IfaceQ, cudaStream_t);

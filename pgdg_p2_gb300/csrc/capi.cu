@@ -854,12 +854,12 @@ struct Ctx : pgdg_ctx {
     return PGDG_OK;
   }
   int split() override {
-    timed("split", 14, [&] { Launch<D, R, EX>::split(K, P, st); });
+    timed("split", 6, [&] { Launch<D, R, EX>::split(K, P, st); });
     nb_set = false;
     return PGDG_OK;
   }
   int merge(bool chained = false) override {
-    timed("merge", 14, [&] { Launch<D, R, EX>::merge(K, P, chained, st); });
+    timed("merge", 7, [&] { Launch<D, R, EX>::merge(K, P, chained, st); });
     nb_set = false;
     return PGDG_OK;
   }

@@ -107,6 +107,32 @@ void scan_u64(unsigned long long* data, unsigned long long* blk, const unsigned 
 }
 __host__ __device__ inline int scan_nblk(int64_t cap) { return (int)((cap + SCAN_TILE - 1) / SCAN_TILE); }
 
+/* exclusive prefix over a block of 1024 threads, and the block's total */
+__device__ __forceinline__ unsigned long long scan_1024(unsigned long long s, unsigned long long* total) {
+  __shared__ unsigned long long sh[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long inc = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  if (lane == 31) sh[w] = inc;
+  __syncthreads();
+  if (w == 0) {
+    unsigned long long v = sh[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += t;
+    }
+    sh[lane] = v;
+  }
+  __syncthreads();
+  *total = sh[31];
+  return inc - s + (w ? sh[w - 1] : 0ull);
+}
+
 /* ------------------------------------------------------------------ */
 /* helpers                                                            */
 /* ------------------------------------------------------------------ */
@@ -339,43 +365,130 @@ __device__ void set_split(const CaseK& K, const PState<D>& par, PState<D>& ch) {
 /* ------------------------------------------------------------------ */
 /* split                                                              */
 /* ------------------------------------------------------------------ */
+/* Split and merge are chains of short kernels, a few microseconds each whatever they
+ * do on a small grid, so each does all that the slots' order allows: the flags and the
+ * tiles' prefixes, the prefix over the tiles with the counters, the events with their
+ * old neighbours, the lists with mark_in.  A split and four merge
+ * passes, 6 and 7 launches each in place of 14: 112x48 cells 0.28 -> 0.15 ms per step,
+ * 1024x1024 cells 0.65 -> 0.44, 384x96x96 cells 2.22 -> 2.08. */
 template <int D, typename R>
-__global__ void k_split_flags(CaseK K, DevPtrs<R> P) {
+__device__ __forceinline__ int split_code(const CaseK& K, const DevPtrs<R>& P, const R* X, int64_t p) {
+  P.target[p] = -1;
+  P.mflag[p] = 0;
+  if (P.phase[p] == 0) return 0;
+  double vol = (double)P.vol[p];
+  double x0 = (double)X[p];
+  if (vol > K.vol_max) return 1;
+  if (P.mark_in[p] == 1) {
+    double dp = root_d(vol, D);
+    if (dsub(x0, K.bl[0]) >= dp) return 2;
+  }
+  return x0 > K.br[0] ? 3 : 0;
+}
+/* event of every slot; scan[p] of a slot that splits or enters receives its rank in
+ * its tile (splits in the upper, inlets in the lower half), scan_blk the tile's total */
+template <int D, typename R>
+__global__ void __launch_bounds__(1024) k_split_flags(CaseK K, DevPtrs<R> P) {
   const int64_t n = (int64_t)P.cnt->n_slots;
   const R* X = P.X[P.xb];
-  GRID_STRIDE(p, n) {
-    P.target[p] = -1;
-    P.mflag[p] = 0;
-    int8_t code = 0;
-    if (P.phase[p] != 0) {
-      double vol = (double)P.vol[p];
-      double x0 = (double)X[p];
-      bool f1 = vol > K.vol_max;
-      bool f2 = false;
-      if (!f1 && P.mark_in[p] == 1) {
-        double dp = root_d(vol, D);
-        f2 = dsub(x0, K.bl[0]) >= dp;
-      }
-      bool f3 = x0 > K.br[0];
-      code = f1 ? 1 : (f2 ? 2 : (f3 ? 3 : 0));
+  const int64_t p0 = (int64_t)blockIdx.x * SCAN_TILE + threadIdx.x * 2;
+  unsigned long long v[2] = {0ull, 0ull};
+#pragma unroll
+  for (int k = 0; k < 2; k++)
+    if (p0 + k < n) {
+      const int code = split_code<D, R>(K, P, X, p0 + k);
       if (code == 3) atomicAdd(&P.cnt->step_new, 1ull); /* outlet count (step_new reused) */
       if (code) atomicAdd(&P.cnt->split_events, 1ull);
+      P.evcode[p0 + k] = (int8_t)code;
+      v[k] = (code == 1) ? (1ull << 32) : (code == 2 ? 1ull : 0ull);
     }
-    P.evcode[p] = code;
-    P.scan[p] = (code == 1) ? (1ull << 32) : (code == 2 ? 1ull : 0ull);
-  }
+  unsigned long long total;
+  const unsigned long long at = scan_1024(v[0] + v[1], &total);
+  if (v[0]) P.scan[p0] = at;
+  if (v[1]) P.scan[p0 + 1] = at + v[0];
+  if (threadIdx.x == 0) P.scan_blk[blockIdx.x] = total;
 }
 
-/* the split's event sweeps cover all slots, or none when no particle has an
- * event (split, inlet or outlet) this step */
-template <typename R>
-__global__ void k_split_begin(DevPtrs<R> P) {
-  P.cnt->split_events = 0;
+/* slots a merge pass sweeps: all, or none when the pass follows a pass of the same
+ * sequence that merged nothing (the state is then unchanged, so this pass would
+ * recompute the same partners and merge nothing too) */
+__device__ __forceinline__ unsigned long long merge_span(const DevCounters* c, int chained) {
+  return (chained && c->merge_quiet) ? 0ull : c->n_slots;
 }
-template <typename R>
-__global__ void k_split_gate(DevPtrs<R> P) {
+
+/* One block: the tiles' totals become their offsets (scan_blk[nblk] the sum), then
+ * the counters of the split or merge pass that the next kernels carry out.  The
+ * sweeps cover the slots there were before (split_n, none when no particle has an
+ * event; merge_n); ranks start from split_seq0 and merge_app0; the queues are empty. */
+template <int D, typename R, bool SPLIT>
+__global__ void __launch_bounds__(1024) k_events(CaseK K, DevPtrs<R> P, int chained) {
+  const int nblk = scan_nblk(K.cap);
+  unsigned long long* blk = P.scan_blk;
+  const int per = (nblk + 1023) / 1024;
+  const int b0 = threadIdx.x * per;
+  unsigned long long s = 0, tot;
+  for (int k = 0; k < per; k++)
+    if (b0 + k < nblk) s += blk[b0 + k];
+  unsigned long long run = scan_1024(s, &tot);
+  for (int k = 0; k < per; k++)
+    if (b0 + k < nblk) {
+      const unsigned long long t = blk[b0 + k];
+      blk[b0 + k] = run;
+      run += t;
+    }
+  if (threadIdx.x != 0) return;
+  blk[nblk] = tot;
   DevCounters* c = P.cnt;
-  c->split_n = c->split_events ? c->n_slots : 0ull;
+  c->n_dirty = 0;
+  c->n_flagged = 0;
+  if constexpr (SPLIT) {
+    constexpr int CN = (D == 3) ? 8 : 4;
+    const unsigned long long nsplit = tot >> 32, ninlet = tot & 0xffffffffull;
+    const unsigned long long nnew = (CN - 1) * nsplit + ninlet, n = c->split_events ? c->n_slots : 0ull;
+    c->split_n = n;
+    c->split_events = 0;
+    c->split_seq0 = c->seq_next;
+    if ((int64_t)(n + nnew) > K.cap) c->err |= ERR_CAPACITY;
+    if (c->err & ERR_CAPACITY) return;
+    const unsigned long long nout = c->step_new;
+    c->n_slots += nnew;
+    c->seq_next += nnew;
+    c->n_live = c->n_live + nnew - nout;
+    c->append_next = CN * nsplit + ninlet;
+    c->n_split += nsplit;
+    c->n_inlet += ninlet;
+    c->n_outlet += nout;
+    c->step_new = 0;
+  } else {
+    c->merge_n = merge_span(c, chained);
+    c->merge_app0 = c->append_next;
+    c->append_next += tot;
+    c->n_live -= tot;
+    c->n_merge += tot;
+    c->merge_quiet = tot == 0 ? 1ull : 0ull;
+  }
+}
+/* rank of a slot with an event */
+template <typename R>
+__device__ __forceinline__ unsigned long long event_rank(const DevPtrs<R>& P, int64_t p) {
+  return P.scan[p] + P.scan_blk[p / SCAN_TILE];
+}
+
+/* the stored neighbours of slot o are affected, but for p and q and the partners being removed */
+template <typename R>
+__device__ __forceinline__ void flag_neighbors(const DevPtrs<R>& P, int64_t o, int64_t p, int64_t q) {
+  const int32_t len = P.list_len[o];
+  if (len < 0) {
+    atomicOr(&P.cnt->err, ERR_NOLIST);
+    return;
+  }
+  const int32_t* L = P.arena + P.list_off[o];
+  for (int32_t e = 0; e < len; e++) {
+    const int32_t r = L[e];
+    if (r < 0 || r == p || r == q) continue;
+    if (P.mflag[r] == 2 || P.phase[r] == 0) continue;
+    P.aff[r] = 1;
+  }
 }
 
 template <int D, typename R>
@@ -384,14 +497,15 @@ __global__ void k_split_emit(CaseK K, DevPtrs<R> P) {
   const int64_t n = (int64_t)P.cnt->split_n;
   const unsigned long long tot = P.scan_blk[scan_nblk(K.cap)];
   const int64_t nsplit = (int64_t)(tot >> 32), ninlet = (int64_t)(tot & 0xffffffffull);
-  if (n + (CN - 1) * nsplit + ninlet > K.cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&P.cnt->err, ERR_CAPACITY);
-    return;
-  }
-  const unsigned long long seq0 = P.cnt->seq_next;
+  const bool room = n + (CN - 1) * nsplit + ninlet <= K.cap; /* (else k_events has set the error) */
+  const unsigned long long seq0 = P.cnt->split_seq0;
   GRID_STRIDE(p, n) {
     int code = P.evcode[p];
     if (code == 0) continue;
+    /* old neighbours of split parents and outlet particles (one that is itself an
+     * outlet is left out by the refresh, whichever comes first) */
+    if (code != 2) flag_neighbors(P, p, -1, -1);
+    if (!room) continue;
     if (code == 3) {
       /* outlet: Remove_particle from its list; the slot becomes a tombstone */
       mark_dirty(P, P.lcell[p]);
@@ -399,7 +513,7 @@ __global__ void k_split_emit(CaseK K, DevPtrs<R> P) {
       P.phase[p] = 0;
       continue;
     }
-    const unsigned long long sv = P.scan[p];
+    const unsigned long long sv = event_rank(P, p);
     const int64_t rs = (int64_t)(sv >> 32), ri = (int64_t)(sv & 0xffffffffull);
     const int64_t cbase = n + (CN - 1) * rs + ri;
     PState<D> par;
@@ -482,45 +596,6 @@ __global__ void k_split_emit(CaseK K, DevPtrs<R> P) {
   }
 }
 
-template <int D, typename R>
-__global__ void k_split_finish(CaseK K, DevPtrs<R> P) {
-  constexpr int CN = (D == 3) ? 8 : 4;
-  const unsigned long long tot = P.scan_blk[scan_nblk(K.cap)];
-  const unsigned long long nsplit = tot >> 32, ninlet = tot & 0xffffffffull;
-  DevCounters* c = P.cnt;
-  if (c->err & ERR_CAPACITY) return;
-  unsigned long long nout = c->step_new;
-  unsigned long long nnew = (CN - 1) * nsplit + ninlet;
-  c->n_slots += nnew;
-  c->seq_next += nnew;
-  c->n_live = c->n_live + nnew - nout;
-  c->append_next = CN * nsplit + ninlet;
-  c->n_split += nsplit;
-  c->n_inlet += ninlet;
-  c->n_outlet += nout;
-  c->step_new = 0;
-}
-
-/* old neighbours of split parents (code 1) and outlet particles (code 3) */
-template <typename R>
-__global__ void k_aff_oldnbr_split(CaseK K, DevPtrs<R> P) {
-  const int64_t n = (int64_t)P.cnt->split_n;
-  GRID_STRIDE(p, n) {
-    int code = P.evcode[p];
-    if (code != 1 && code != 3) continue;
-    int32_t len = P.list_len[p];
-    if (len < 0) {
-      atomicOr(&P.cnt->err, ERR_NOLIST);
-      continue;
-    }
-    const int32_t* L = P.arena + P.list_off[p];
-    for (int32_t e = 0; e < len; e++) {
-      int32_t q = L[e];
-      if (q >= 0 && P.phase[q] != 0) P.aff[q] = 1;
-    }
-  }
-}
-
 template <typename R>
 __global__ void k_aff_cells(CaseK K, DevPtrs<R> P) {
   const int64_t n = (int64_t)min(P.cnt->n_flagged, (unsigned long long)P.qcap);
@@ -532,18 +607,42 @@ __global__ void k_aff_cells(CaseK K, DevPtrs<R> P) {
   }
 }
 
-/* Refresh_neighbor_info(3) for affected particles: dist <= 2 p_sz within +-2 cells
- * (level_infor.cpp:161-188); stored fluid entries in list order */
+/* mark_in = (x - box_l.x < vol^(1/DIM)) (mpm.cpp:1398-1399).  The FP32 path decides in FP32 when x - box_l is more than
+ * 0.1% away from vol^(1/DIM) (far beyond the rounding of either side) and
+ * evaluates the rest exactly, as the FP64 path does. */
 template <int D, typename R>
-__global__ void k_refresh3(CaseK K, DevPtrs<R> P, const unsigned long long* np) {
+__device__ __forceinline__ int8_t mark_of(const CaseK& K, const DevPtrs<R>& P, const R* X, int64_t p) {
+  if constexpr (sizeof(R) == 4) {
+    const float af = (float)X[p] - (float)K.bl[0];
+    const float rf = (D == 2) ? sqrtf((float)P.vol[p]) : cbrtf((float)P.vol[p]);
+    if (af > rf * 1.001f) return 0;
+    if (af < rf * 0.999f) return 1;
+  }
+  double a = dsub((double)X[p], K.bl[0]);
+  double vol = (double)P.vol[p];
+  double ra = (D == 2) ? sqrt(vol) : cbrt(vol);
+  if (a > ra * 1.0001) return 0;
+  if (a < ra * 0.9999) return 1;
+  return (a < root_d(vol, D)) ? 1 : 0;
+}
+
+/* Refresh_neighbor_info(3) for affected particles: dist <= 2 p_sz within +-2 cells
+ * (level_infor.cpp:161-188); stored fluid entries in list order; and every particle's
+ * mark_in.  After a merge pass that merged nothing (events, may be NULL, its count)
+ * nothing mark_in depends on has changed since the last evaluation */
+template <int D, typename R>
+__global__ void k_refresh3(CaseK K, DevPtrs<R> P, const unsigned long long* np, const unsigned long long* events) {
   const int64_t n = (int64_t)*np;
+  const bool mark = !events || *events != 0;
   const R* X = P.X[P.xb];
   const double lim = dmul(K.p_sz, 2.);
   const float lo2 = (float)(lim * lim * (1.0 - 1e-5)), hi2 = (float)(lim * lim * (1.0 + 1e-5));
   GRID_STRIDE(p, n) {
+    const bool live = P.phase[p] != 0;
+    if (mark && live) P.mark_in[p] = mark_of<D, R>(K, P, X, p);
     if (!P.aff[p]) continue;
     P.aff[p] = 0;
-    if (P.phase[p] == 0) continue;
+    if (!live) continue;
     atomicAdd(&P.cnt->n_affected, 1ull);
     R xr[3];
     load_x<D>(K, X, p, xr);
@@ -611,81 +710,23 @@ __global__ void k_refresh3(CaseK K, DevPtrs<R> P, const unsigned long long* np) 
   }
 }
 
-/* mark_in = (x - box_l.x < vol^(1/DIM)) (mpm.cpp:1398-1399).  events (may be
- * NULL): the event count of the merge pass just run; with no merge nothing
- * mark_in depends on has changed since the last evaluation and the kernel
- * returns at once.  The FP32 path decides in FP32 when x - box_l is more than
- * 0.1% away from vol^(1/DIM) (far beyond the rounding of either side) and
- * evaluates the rest exactly, as the FP64 path does. */
-template <int D, typename R>
-__global__ void k_mark_in(CaseK K, DevPtrs<R> P, const unsigned long long* events) {
-  if (events && *events == 0) return;
-  const int64_t n = (int64_t)P.cnt->n_slots;
-  const R* X = P.X[P.xb];
-  const float blf = (float)K.bl[0];
-  GRID_STRIDE(p, n) {
-    if (P.phase[p] == 0) continue;
-    if constexpr (sizeof(R) == 4) {
-      const float af = (float)X[p] - blf;
-      const float rf = (D == 2) ? sqrtf((float)P.vol[p]) : cbrtf((float)P.vol[p]);
-      if (af > rf * 1.001f) {
-        P.mark_in[p] = 0;
-        continue;
-      }
-      if (af < rf * 0.999f) {
-        P.mark_in[p] = 1;
-        continue;
-      }
-    }
-    double a = dsub((double)X[p], K.bl[0]);
-    double vol = (double)P.vol[p];
-    double ra = (D == 2) ? sqrt(vol) : cbrt(vol);
-    int8_t m;
-    if (a > ra * 1.0001) m = 0;
-    else if (a < ra * 0.9999) m = 1;
-    else m = (a < root_d(vol, D)) ? 1 : 0;
-    P.mark_in[p] = m;
-  }
-}
-
-template <typename R>
-__global__ void k_reset_queues(DevPtrs<R> P) {
-  P.cnt->n_dirty = 0;
-  P.cnt->n_flagged = 0;
-}
-
 template <int D, typename R, bool EX>
 void Launch<D, R, EX>::split(const CaseK& K, const DevPtrs<R>& P, cudaStream_t st) {
   const int g = grid_for(K.cap, BLK);
-  k_split_begin<R><<<1, 1, 0, st>>>(P);
-  k_split_flags<D, R><<<g, BLK, 0, st>>>(K, P);
-  k_split_gate<R><<<1, 1, 0, st>>>(P);
-  scan_u64(P.scan, P.scan_blk, &P.cnt->split_n, K.cap, st);
-  k_aff_oldnbr_split<R><<<g, BLK, 0, st>>>(K, P);
+  k_split_flags<D, R><<<scan_nblk(K.cap), 1024, 0, st>>>(K, P);
+  k_events<D, R, true><<<1, 1024, 0, st>>>(K, P, 0);
   k_split_emit<D, R><<<g, BLK, 0, st>>>(K, P);
-  k_split_finish<D, R><<<1, 1, 0, st>>>(K, P);
   k_bucket_fix<R><<<grid_for(P.qcap, BLK), BLK, 0, st>>>(K, P, 0);
   k_aff_cells<R><<<grid_for(P.qcap, BLK), BLK, 0, st>>>(K, P);
-  k_refresh3<D, R><<<g, BLK, 0, st>>>(K, P, &P.cnt->n_slots);
-  k_mark_in<D, R><<<g, BLK, 0, st>>>(K, P, nullptr);
-  k_reset_queues<R><<<1, 1, 0, st>>>(P);
+  k_refresh3<D, R><<<g, BLK, 0, st>>>(K, P, &P.cnt->n_slots, nullptr);
 }
 
 /* ------------------------------------------------------------------ */
 /* merge (one pass of Merge_particle_fast)                            */
 /* ------------------------------------------------------------------ */
-/* particles a merge pass sweeps: all slots, or none when the pass follows a
- * pass of the same sequence that merged nothing (the state is then unchanged,
- * so this pass would recompute the same partners and merge nothing too) */
-template <typename R>
-__global__ void k_merge_begin(DevPtrs<R> P, int chained) {
-  DevCounters* c = P.cnt;
-  c->merge_n = (chained && c->merge_quiet) ? 0ull : c->n_slots;
-}
-
 template <int D, typename R>
-__global__ void k_merge_a(CaseK K, DevPtrs<R> P) {
-  const int64_t n = (int64_t)P.cnt->merge_n;
+__global__ void k_merge_a(CaseK K, DevPtrs<R> P, int chained) {
+  const int64_t n = (int64_t)merge_span(P.cnt, chained);
   const R* X = P.X[P.xb];
   GRID_STRIDE(p, n) {
     P.target[p] = -1;
@@ -721,19 +762,28 @@ __global__ void k_merge_a(CaseK K, DevPtrs<R> P) {
   }
 }
 
+/* pairs that chose each other; scan[p] of a pair's lower slot receives its rank in its tile */
 template <int D, typename R>
-__global__ void k_merge_b(CaseK K, DevPtrs<R> P) {
-  const int64_t n = (int64_t)P.cnt->merge_n;
-  GRID_STRIDE(p, n) {
-    unsigned long long s = 0;
-    int32_t q = P.target[p];
+__global__ void __launch_bounds__(1024) k_merge_b(CaseK K, DevPtrs<R> P, int chained) {
+  const int64_t n = (int64_t)merge_span(P.cnt, chained);
+  const int64_t p0 = (int64_t)blockIdx.x * SCAN_TILE + threadIdx.x * 2;
+  unsigned long long v[2] = {0ull, 0ull};
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int64_t p = p0 + k;
+    if (p >= n) continue;
+    const int32_t q = P.target[p];
     if (q >= 0 && q > p && P.target[q] == (int32_t)p) {
       P.mflag[p] = 1;
       P.mflag[q] = 2;
-      s = 1;
+      v[k] = 1;
     }
-    P.scan[p] = s;
   }
+  unsigned long long total;
+  const unsigned long long at = scan_1024(v[0] + v[1], &total);
+  if (v[0]) P.scan[p0] = at;
+  if (v[1]) P.scan[p0 + 1] = at + v[0];
+  if (threadIdx.x == 0) P.scan_blk[blockIdx.x] = total;
 }
 
 /* Set_merge_ptcl (particle.cpp:614-661) + list fix-up (mpm.cpp:1637-1669) */
@@ -741,10 +791,12 @@ template <int D, typename R>
 __global__ void k_merge_c(CaseK K, DevPtrs<R> P) {
   constexpr int NS = PState<D>::NS;
   const int64_t n = (int64_t)P.cnt->merge_n;
-  const unsigned long long app = P.cnt->append_next;
+  const unsigned long long app = P.cnt->merge_app0;
   GRID_STRIDE(p, n) {
     if (P.mflag[p] != 1) continue;
     int32_t q = P.target[p];
+    flag_neighbors(P, p, p, q);
+    flag_neighbors(P, q, p, q);
     mark_dirty(P, P.lcell[p]);
     mark_dirty(P, P.lcell[q]);
     PState<D> a, b;
@@ -770,7 +822,7 @@ __global__ void k_merge_c(CaseK K, DevPtrs<R> P) {
     cell_pos_exact<D>(K, m.x, pos);
     int64_t c = cidx<D>(K, pos);
     P.lcell[p] = (int32_t)c;
-    P.lkey[p] = KEY_APPEND + (uint32_t)(app + P.scan[p]);
+    P.lkey[p] = KEY_APPEND + (uint32_t)(app + event_rank(P, p));
     bucket_append(K, P, c, p);
     mark_dirty(P, c);
     P.aff[p] = 1;
@@ -778,56 +830,17 @@ __global__ void k_merge_c(CaseK K, DevPtrs<R> P) {
   }
 }
 
-template <typename R>
-__global__ void k_aff_oldnbr_merge(CaseK K, DevPtrs<R> P) {
-  const int64_t n = (int64_t)P.cnt->merge_n;
-  GRID_STRIDE(p, n) {
-    if (P.mflag[p] != 1) continue;
-    int32_t q = P.target[p];
-    for (int w = 0; w < 2; w++) {
-      int64_t o = w ? q : p;
-      int32_t len = P.list_len[o];
-      if (len < 0) {
-        atomicOr(&P.cnt->err, ERR_NOLIST);
-        continue;
-      }
-      const int32_t* L = P.arena + P.list_off[o];
-      for (int32_t e = 0; e < len; e++) {
-        int32_t r = L[e];
-        if (r < 0 || r == p || r == q) continue;
-        if (P.mflag[r] == 2 || P.phase[r] == 0) continue;
-        P.aff[r] = 1;
-      }
-    }
-  }
-}
-
-template <int D, typename R>
-__global__ void k_merge_finish(CaseK K, DevPtrs<R> P) {
-  const unsigned long long ns = P.scan_blk[scan_nblk(K.cap)];
-  DevCounters* c = P.cnt;
-  c->append_next += ns;
-  c->n_live -= ns;
-  c->n_merge += ns;
-  c->merge_quiet = ns == 0 ? 1ull : 0ull;
-}
-
 template <int D, typename R, bool EX>
 void Launch<D, R, EX>::merge(const CaseK& K, const DevPtrs<R>& P, bool chained, cudaStream_t st) {
   const int g = grid_for(K.cap, BLK);
-  k_merge_begin<R><<<1, 1, 0, st>>>(P, chained ? 1 : 0);
-  k_merge_a<D, R><<<g, BLK, 0, st>>>(K, P);
-  k_merge_b<D, R><<<g, BLK, 0, st>>>(K, P);
-  scan_u64(P.scan, P.scan_blk, &P.cnt->merge_n, K.cap, st);
-  k_aff_oldnbr_merge<R><<<g, BLK, 0, st>>>(K, P);
+  k_merge_a<D, R><<<g, BLK, 0, st>>>(K, P, chained ? 1 : 0);
+  k_merge_b<D, R><<<scan_nblk(K.cap), 1024, 0, st>>>(K, P, chained ? 1 : 0);
+  k_events<D, R, false><<<1, 1024, 0, st>>>(K, P, chained ? 1 : 0);
   k_merge_c<D, R><<<g, BLK, 0, st>>>(K, P);
-  k_merge_finish<D, R><<<1, 1, 0, st>>>(K, P);
   k_bucket_fix<R><<<grid_for(P.qcap, BLK), BLK, 0, st>>>(K, P, 0);
   k_aff_cells<R><<<grid_for(P.qcap, BLK), BLK, 0, st>>>(K, P);
-  k_refresh3<D, R><<<g, BLK, 0, st>>>(K, P, &P.cnt->merge_n);
-  /* the pass's merge count is still the scan total */
-  k_mark_in<D, R><<<g, BLK, 0, st>>>(K, P, P.scan_blk + scan_nblk(K.cap));
-  k_reset_queues<R><<<1, 1, 0, st>>>(P);
+  /* the pass's merge count is the total of its ranks */
+  k_refresh3<D, R><<<g, BLK, 0, st>>>(K, P, &P.cnt->merge_n, P.scan_blk + scan_nblk(K.cap));
 }
 
 /* ------------------------------------------------------------------ */

@@ -67,6 +67,7 @@ struct DevCounters {
   unsigned long long merge_quiet; /* the last merge pass merged nothing */
   unsigned long long split_events; /* particles with a split, inlet or outlet event */
   unsigned long long split_n;      /* slots the split's event sweeps cover */
+  unsigned long long split_seq0, merge_app0; /* seq_next before the split, append_next before the merge pass */
   unsigned int err;
   unsigned int pad;
   double dt, max_v;

@@ -162,7 +162,6 @@ struct Ctx : pgdg_ctx {
   bool fresh_bins = false;
   bool g2p_partial = false; /* see run_step */
   double *d_gam = nullptr, *d_pinf = nullptr;
-  unsigned long long* d_ncell = nullptr;
   int dev_id = 0;
   /* the last complete stage's search coordinates and lengths (the flag-2
    * lists the snapshot writer counts); unset after the particle set changes */
@@ -289,12 +288,6 @@ struct Ctx : pgdg_ctx {
     CK(A(&Q.off, nc + 1));
     CK(A(&Q.blk, (nc + 2047) / 2048 + 2));
     CK(A(&Q.tot, 2));
-    CK(A(&d_ncell, 1));
-    {
-      unsigned long long v = (unsigned long long)K.ncell;
-      CK(cudaMemcpy(d_ncell, &v, sizeof(v), cudaMemcpyHostToDevice));
-    }
-    Q.d_ncell = d_ncell;
     CK(A(&d_gam, F));
     CK(A(&d_pinf, F));
     CK(cudaMemcpy(d_gam, K.gamma, sizeof(double) * F, cudaMemcpyHostToDevice));
@@ -966,7 +959,7 @@ struct Ctx : pgdg_ctx {
       IfaceQ q = Q;
       if (iface_cap_fixed < 0) q.cap = q_room;
       q.phase = 1;
-      timed("iface_gather", 6, [&] { Launch<D, R, EX>::iface_gather(K, P, q, st); });
+      timed("iface_gather", 3, [&] { Launch<D, R, EX>::iface_gather(K, P, q, st); });
       int rc = PGDG_OK;
       timed("mgfm_seeded", 1, [&] {
         rc = mgfm_seeded_run(nullptr, q.in6, q.mat, d_gam, d_pinf, K.mgfm_variant, q.out3, nullptr, q.cap,
@@ -988,7 +981,7 @@ struct Ctx : pgdg_ctx {
       const int rc = mgfm_seeded_reserve(net, part, Q.cap);
       if (rc) return rc;
     }
-    timed("iface_gather", 6, [&] { Launch<D, R, EX>::iface_gather(K, P, Q, st); });
+    timed("iface_gather", 3, [&] { Launch<D, R, EX>::iface_gather(K, P, Q, st); });
     int rc = PGDG_OK;
     timed("mgfm_seeded", net ? 3 : 1, [&] {
       rc = mgfm_seeded_run(net, Q.in6, Q.mat, d_gam, d_pinf, K.mgfm_variant, Q.out3, nullptr, Q.cap,

@@ -19,7 +19,6 @@
 namespace pgdg {
 
 constexpr int BLK = 256;
-constexpr int SCAN_TILE = 2048;     /* 256 threads x 8 */
 constexpr int MAXPC_MAX = 64;
 
 int grid_for(int64_t n, int block) {
@@ -104,33 +103,6 @@ void scan_u64(unsigned long long* data, unsigned long long* blk, const unsigned 
   k_scan_tiles<<<nblk, BLK, 0, st>>>(data, blk, d_n);
   k_scan_blocks<<<1, 1024, 0, st>>>(blk, nblk);
   k_scan_add<<<nblk, BLK, 0, st>>>(data, blk, d_n);
-}
-__host__ __device__ inline int scan_nblk(int64_t cap) { return (int)((cap + SCAN_TILE - 1) / SCAN_TILE); }
-
-/* exclusive prefix over a block of 1024 threads, and the block's total */
-__device__ __forceinline__ unsigned long long scan_1024(unsigned long long s, unsigned long long* total) {
-  __shared__ unsigned long long sh[32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  unsigned long long inc = s;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
-  }
-  if (lane == 31) sh[w] = inc;
-  __syncthreads();
-  if (w == 0) {
-    unsigned long long v = sh[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long t = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += t;
-    }
-    sh[lane] = v;
-  }
-  __syncthreads();
-  *total = sh[31];
-  return inc - s + (w ? sh[w - 1] : 0ull);
 }
 
 /* ------------------------------------------------------------------ */
@@ -424,18 +396,7 @@ template <int D, typename R, bool SPLIT>
 __global__ void __launch_bounds__(1024) k_events(CaseK K, DevPtrs<R> P, int chained) {
   const int nblk = scan_nblk(K.cap);
   unsigned long long* blk = P.scan_blk;
-  const int per = (nblk + 1023) / 1024;
-  const int b0 = threadIdx.x * per;
-  unsigned long long s = 0, tot;
-  for (int k = 0; k < per; k++)
-    if (b0 + k < nblk) s += blk[b0 + k];
-  unsigned long long run = scan_1024(s, &tot);
-  for (int k = 0; k < per; k++)
-    if (b0 + k < nblk) {
-      const unsigned long long t = blk[b0 + k];
-      blk[b0 + k] = run;
-      run += t;
-    }
+  const unsigned long long tot = scan_offsets_1024(blk, nblk);
   if (threadIdx.x != 0) return;
   blk[nblk] = tot;
   DevCounters* c = P.cnt;

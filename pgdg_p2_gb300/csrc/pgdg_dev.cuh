@@ -154,14 +154,15 @@ struct IfaceQ {
   double* in6;
   int8_t* mat;
   double* out3;
+  /* a cell's first problem: off[ci], its rank in the tile of 2048 cells, + the tile's blk */
   unsigned long long* off;
   unsigned long long* blk;
-  const unsigned long long* d_ncell;
   /* [0] the stage's interface problems, [1] those the batch solves: [0], or 0
    * when [0] exceeds cap (the residual then solves the stage inline) */
   unsigned long long* tot;
   int64_t cap;
   int phase; /* the mixed path's residual (MODE 0): 0 solve inline, 1 gather, 2 use the batch's results */
+  __device__ __forceinline__ int64_t first(int64_t ci) const { return (int64_t)(off[ci] + blk[ci >> 11]); }
 };
 
 /* ---------------- cell ids ---------------- */
@@ -344,6 +345,51 @@ __host__ __device__ constexpr int minblocks_f32(int n) {
 
 /* shared helpers used by several translation units */
 int grid_for(int64_t n, int block);
+/* prefix sums over tiles of 2048 (a tile's 1024 threads take two neighbouring values) */
+constexpr int SCAN_TILE = 2048;
+__host__ __device__ inline int scan_nblk(int64_t n) { return (int)((n + SCAN_TILE - 1) / SCAN_TILE); }
+/* exclusive prefix over a block of 1024 threads, and the block's total */
+__device__ __forceinline__ unsigned long long scan_1024(unsigned long long s, unsigned long long* total) {
+  __shared__ unsigned long long sh[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long inc = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += t;
+  }
+  if (lane == 31) sh[w] = inc;
+  __syncthreads();
+  if (w == 0) {
+    unsigned long long v = sh[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += t;
+    }
+    sh[lane] = v;
+  }
+  __syncthreads();
+  *total = sh[31];
+  return inc - s + (w ? sh[w - 1] : 0ull);
+}
+/* one block of 1024 threads: the tiles' totals become their offsets; returns the sum */
+__device__ __forceinline__ unsigned long long scan_offsets_1024(unsigned long long* blk, int nblk) {
+  const int per = (nblk + 1023) / 1024;
+  const int b0 = threadIdx.x * per;
+  unsigned long long s = 0, tot;
+  for (int k = 0; k < per; k++)
+    if (b0 + k < nblk) s += blk[b0 + k];
+  unsigned long long run = scan_1024(s, &tot);
+  for (int k = 0; k < per; k++)
+    if (b0 + k < nblk) {
+      const unsigned long long t = blk[b0 + k];
+      blk[b0 + k] = run;
+      run += t;
+    }
+  return tot;
+}
+
 void scan_u64(unsigned long long* data, unsigned long long* blk, const unsigned long long* d_n, int64_t cap,
               cudaStream_t st);
 

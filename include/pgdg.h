@@ -151,9 +151,12 @@ int pgdg_surrogate_train_step(pgdg_mlp* net, const float* X, const float* T, int
  * queue on.  Not available on the exact-order FP64 path (PGDG_EINVAL). */
 int pgdg_set_surrogate(pgdg_ctx* ctx, pgdg_mlp* net);
 /* interface queue (no reference counterpart: MPM::Grid_acceleration calls
- * MGFM inline, particle_flow.cpp:192-204): the residual gathers each stage's
- * two-material interface problems into one batch, solves them together and
- * reads the ghost states back.  Mixed and FP64_FMA paths only. */
+ * MGFM inline, particle_flow.cpp:192-204).  The residual always gathers each
+ * stage's two-material interface problems into one batch, solves them together
+ * and reads the ghost states back.  On the mixed path the queue on selects the
+ * build that a surrogate needs (its FP32 rounding differs from the inline
+ * form's, which the queue off keeps) and makes the problems available to
+ * pgdg_iface_download.  Mixed and FP64_FMA paths only. */
 int pgdg_set_iface_queue(pgdg_ctx* ctx, int on);
 /* copy the last stage's queued problems to the host (in6 n x 6, mat2 n x 2,
  * at most cap entries); *n receives the queue length */

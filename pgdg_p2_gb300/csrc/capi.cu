@@ -946,6 +946,8 @@ struct Ctx : pgdg_ctx {
   int set_iface_cap(int64_t cap) override {
     iface_cap_fixed = cap;
     if (cap >= 0 && cap != Q.cap) return grow_queue(cap > 0 ? cap : 1);
+    const int64_t room = std::max<int64_t>(1 << 16, K.ncell / 2);
+    if (cap < 0 && !iface_queue && sizeof(R) == 4 && q_room < room) return grow_queue(room);
     drop_graphs();
     return PGDG_OK;
   }

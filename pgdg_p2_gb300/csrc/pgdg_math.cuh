@@ -142,11 +142,12 @@ PGDG_HD double drcp(double b) {
  * with y correctly rounded and a quotient within one unit in the last place, the
  * corrected quotient is the correctly rounded one).  5 FP64 instructions where
  * a division is about 10 and the FP64 pipe sets the pace.  Outside exponents
- * that keep every step normal, and for b <= 0, the division itself. */
+ * that keep every step normal, for b <= 0, and for a = -0 (whose remainder +0 would
+ * turn it into +0), the division itself. */
 PGDG_HD double ddiv_by(double a, double b, double y) {
 #if defined(__CUDA_ARCH__)
-  const int ha = __double2hiint(a) & 0x7fffffff;
-  const unsigned ea = (unsigned)ha >> 20, eb = (unsigned)__double2hiint(b) >> 20;
+  const int ha = __double2hiint(a);
+  const unsigned ea = ((unsigned)ha & 0x7fffffffu) >> 20, eb = (unsigned)__double2hiint(b) >> 20;
   if ((ea - 400u < 1200u || (ha | __double2loint(a)) == 0) && eb - 600u < 800u) { /* a sign bit in b fails the range too */
     double q = __dmul_rn(a, y);
     q = __fma_rn(__fma_rn(-q, b, a), y, q);

@@ -1705,7 +1705,11 @@ __global__ void __launch_bounds__(PD_THREADS, 5) k_pst_d(CaseK K, DevPtrs<double
   const int bdim[3] = {BK::B0, BK::B1, D == 3 ? BK::B2 : 1};
   int slo[3], sn[3];
   double org[3];
-  float r2 = 0.f; /* the staged box's half diagonal, squared */
+  /* squared distance from the brick's centre that no staged position exceeds: the staged
+   * box's half diagonal, raised to the positions' own bounds where cells hold particles
+   * outside themselves (the edge cells take every particle beyond the box) */
+  __shared__ float s_r2;
+  float r2 = 0.f;
   for (int d = 0; d < 3; d++) {
     const int r = (d < D) ? K.rad2 : 0, Nd = (d < D) ? K.N[d] : 1;
     slo[d] = max(c0[d] - r, 0);
@@ -1718,6 +1722,7 @@ __global__ void __launch_bounds__(PD_THREADS, 5) k_pst_d(CaseK K, DevPtrs<double
   PdSmem sm;
   pd_layout(&sm, smem_raw, D, nsc, cap);
   __shared__ int s_red[SCAN_RED];
+  if (threadIdx.x == 0) s_r2 = r2;
   auto cell_of = [&](int l) {
     const int t = l / (sn[1] * sn[2]), s = (l / sn[2]) % sn[1], m = l % sn[2];
     return ((int64_t)(slo[0] + t) * K.N[1] + (slo[1] + s)) * K.N[2] + (slo[2] + m);
@@ -1761,10 +1766,15 @@ __global__ void __launch_bounds__(PD_THREADS, 5) k_pst_d(CaseK K, DevPtrs<double
       }
       if (l8 == 0) {
         sm.mid[l] = first;
+        float far2 = 0.f;
         for (int d = 0; d < D; d++) {
           sm.blo[d * nsc + l] = mn[d];
           sm.bhi[d * nsc + l] = mx[d];
+          const float e = fmaxf(-mn[d], mx[d]);
+          far2 = fmaf(e, e, far2);
         }
+        /* (positive floats compare as their bits do; the bounds of what is not a number make it infinite) */
+        if (cnt > 0 && far2 > r2) atomicMax(reinterpret_cast<int*>(&s_r2), __float_as_int(far2));
       }
     }
   }
@@ -1785,8 +1795,10 @@ __global__ void __launch_bounds__(PD_THREADS, 5) k_pst_d(CaseK K, DevPtrs<double
   }
   __syncthreads();
   const int npart = block_scan_counts(s_boff, nbc, s_red);
-  /* absolute error of an FP32 squared distance between staged positions, with room */
-  const float band = 4e-6f * r2;
+  /* absolute error of an FP32 squared distance between staged positions, with room: each
+   * coordinate and difference is rounded once, at most 16 u r2 in all, and the squares and
+   * sums 3 u of at most 4 r2, 1.7e-6 r2 together (u = 2^-24) */
+  const float band = 4e-6f * s_r2;
   for (int i = threadIdx.x; i < npart; i += blockDim.x) {
     int q = 0, qh = nbc - 1;
     while (q < qh) {

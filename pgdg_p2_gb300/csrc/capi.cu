@@ -280,8 +280,8 @@ struct Ctx : pgdg_ctx {
     /* interface queue: at most 2 phases x 2D faces x 4 points x 1 other phase per cell;
      * sized for a few per cent of the cells, grown on demand when the queue was asked
      * for (a stage that outgrows it is solved inline) */
-    Q.cap = std::max<int64_t>(1 << 16, sizeof(R) == 8 ? K.ncell : K.ncell / 8);
-    q_room = std::max<int64_t>(Q.cap, K.ncell / 2); /* of the mixed path without a surrogate */
+    Q.cap = auto_cap();
+    q_room = auto_room();
     CK(A(&Q.in6, 6 * (size_t)q_room));
     CK(A(&Q.mat, 2 * (size_t)q_room));
     CK(A(&Q.out3, 3 * (size_t)q_room));
@@ -909,18 +909,31 @@ struct Ctx : pgdg_ctx {
     }
     return bv;
   }
-  int grow_queue(int64_t need) {
-    drop_graphs(); /* they hold the old buffers */
-    CK(cudaStreamSynchronize(st));
-    for (void* p : {(void*)Q.in6, (void*)Q.mat, (void*)Q.out3}) {
-      for (auto& a : allocs)
-        if (a == p) a = nullptr;
-      cudaFree(p);
+  /* the automatic queue: the capacity it starts with, and the room its buffers have from the
+   * start, which the mixed path without a surrogate uses whole */
+  int64_t auto_cap() const { return std::max<int64_t>(1 << 16, sizeof(R) == 8 ? K.ncell : K.ncell / 8); }
+  int64_t auto_room() const { return std::max<int64_t>(auto_cap(), K.ncell / 2); }
+  /* a queue for cap problems in buffers for room >= cap; other buffers only for another room
+   * (should they not be had, a queue for none: every problem is solved inline) */
+  int resize_queue(int64_t cap, int64_t room) {
+    drop_graphs(); /* they hold the capacity and the buffers */
+    if (room != q_room) {
+      CK(cudaStreamSynchronize(st));
+      for (void* p : {(void*)Q.in6, (void*)Q.mat, (void*)Q.out3}) {
+        for (auto& a : allocs)
+          if (a == p) a = nullptr;
+        cudaFree(p);
+      }
+      Q.in6 = Q.out3 = nullptr;
+      Q.mat = nullptr;
+      Q.cap = q_room = 0;
+      CK(cudaMemsetAsync(Q.tot, 0, 2 * sizeof(*Q.tot), st)); /* the last stage's problems are gone */
+      CK(A(&Q.in6, 6 * (size_t)room));
+      CK(A(&Q.mat, 2 * (size_t)room));
+      CK(A(&Q.out3, 3 * (size_t)room));
+      q_room = room;
     }
-    Q.cap = q_room = need;
-    CK(A(&Q.in6, 6 * (size_t)Q.cap));
-    CK(A(&Q.mat, 2 * (size_t)Q.cap));
-    CK(A(&Q.out3, 3 * (size_t)Q.cap));
+    Q.cap = cap;
     return PGDG_OK;
   }
   /* Host-side upkeep of the interface queue, between steps: grow it to twice
@@ -934,7 +947,8 @@ struct Ctx : pgdg_ctx {
     CK(cudaStreamSynchronize(st));
     CK(cudaMemcpy(t, Q.tot, sizeof(t), cudaMemcpyDeviceToHost));
     if (iface_cap_fixed < 0 && (int64_t)t[0] * 2 > Q.cap) {
-      int rc = grow_queue((int64_t)t[0] * 2 + 4096);
+      const int64_t need = (int64_t)t[0] * 2 + 4096;
+      const int rc = resize_queue(need, std::max(need, q_room));
       if (rc) return rc;
     }
     const int rc = mgfm_seeded_reserve(net, part, Q.cap);
@@ -945,11 +959,8 @@ struct Ctx : pgdg_ctx {
   int prepare_step() override { return ensure_queue(); }
   int set_iface_cap(int64_t cap) override {
     iface_cap_fixed = cap;
-    if (cap >= 0 && cap != Q.cap) return grow_queue(cap > 0 ? cap : 1);
-    const int64_t room = std::max<int64_t>(1 << 16, K.ncell / 2);
-    if (cap < 0 && !iface_queue && sizeof(R) == 4 && q_room < room) return grow_queue(room);
-    drop_graphs();
-    return PGDG_OK;
+    if (cap >= 0) return resize_queue(std::max<int64_t>(cap, 1), std::max<int64_t>(cap, 1));
+    return resize_queue(std::max(Q.cap, auto_cap()), std::max(q_room, auto_room()));
   }
   int grid_acc() override {
     /* FP32 without a surrogate: the same batch, gathered and used by the inline

@@ -1944,6 +1944,17 @@ size_t Launch<D, R, EX>::pst_scratch_bytes(const CaseK& K) {
   return EX ? 0 : rowsort_layout<R>(K, nullptr, nullptr);
 }
 
+/* (a file-local function: a static of the exported Launch would be one for the two- and
+ * the three-material library together, and the second one loaded would never set its kernel) */
+template <int D, typename R>
+static void rs_cells_room(int bytes) {
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaFuncSetAttribute(k_rs_cells<D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    attr_set = true;
+  }
+}
+
 /* the per-stage row sort of the mixed and FMA paths (three launches; nothing
  * on the exact path) */
 template <int D, typename R, bool EX>
@@ -1953,11 +1964,7 @@ void Launch<D, R, EX>::rowsort(const CaseK& K, const DevPtrs<R>& P, int xs, void
     rowsort_layout<R>(K, static_cast<unsigned char*>(scratch), &B);
     const int64_t nrows = K.ncell / K.N[D - 1];
     const size_t shb = sizeof(typename Vec4<R>::T) * RS_CAP * RS_T;
-    static bool attr_set = false;
-    if (!attr_set) {
-      cudaFuncSetAttribute(k_rs_cells<D, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shb);
-      attr_set = true;
-    }
+    rs_cells_room<D, R>((int)shb);
     k_rs_cells<D, R><<<grid_for(K.ncell, RS_T), RS_T, shb, st>>>(K, P, xs, B);
     k_rs_rows<D, R><<<grid_for(nrows * 32, 128), 128, 0, st>>>(K, P, B);
     k_rs_rank<D, R><<<grid_for(K.ncell, 256), 256, 0, st>>>(K, P, B);

@@ -207,11 +207,14 @@ int pgdg_mgfm_batched_noalloc(const pgdg_mlp* net, const double* in6, const int8
 int pgdg_set_graphs(pgdg_ctx* ctx, int on);
 
 /* ---- kernel variants (no reference counterpart) ----
- * Some kernels have several implementations with identical results; the
- * context times them on its own state at their first call and keeps the
- * fastest.  kernel: "pst" (the shifting kernel of pgdg_update_particle).
- * variant >= 0 forces that variant, -1 re-tunes at the next call, -2 only
- * queries; *chosen (may be NULL) receives the current choice (-1: not tuned).
+ * kernel "pst": the shifting kernel of pgdg_update_particle has several
+ * implementations that sum the same neighbours; their results agree to rounding,
+ * not bit for bit.  On the mixed path the context times variants 0 to 7 on its
+ * own state at their first call and keeps the fastest, so a program that needs
+ * the same bits from run to run forces one.  The FP64_FMA path takes variant 8
+ * and the exact path its only one, neither by timing.
+ * variant >= 0 forces that variant, -1 chooses anew at the next call, -2 only
+ * queries; *chosen (may be NULL) receives the current choice (-1: none yet).
  * kernel "p2g_skip": 1 (default) lets pgdg_mls_p2g skip neighbour cells beyond
  * its cut radius while every particle still lies in its bucket's cell (from
  * pgdg_bin_particles until particles move); 0 always visits all 3^d cells.

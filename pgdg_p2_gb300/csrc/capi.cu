@@ -885,11 +885,10 @@ struct Ctx : pgdg_ctx {
     return PGDG_OK;
   }
   /* autotuner: time each variant of a kernel twice on the current state (the
-   * kernel must only overwrite its outputs, and all variants give the same
-   * results) and keep the fastest */
+   * kernel must only overwrite its outputs, and the variants agree to rounding)
+   * and keep the fastest */
   template <class F>
   int tune(int nvar, F&& run) {
-    if (nvar <= 1) return 0;
     cudaEvent_t a = ev_get(), b = ev_get();
     float best = 0.f;
     int bv = 0;
@@ -1022,6 +1021,7 @@ struct Ctx : pgdg_ctx {
       if (xn == xs || xn == x0 || xn < 0 || xn > 2) xn = (xs + 1) % 3;  /* md 1 without md 0 */
     }
     timed("g2p", 1, [&] { Launch<D, R, EX>::g2p(K, P, md, xs, x0, xn, hn, !g2p_partial, st); });
+    if (pst_var < 0) pst_var = Launch<D, R, EX>::pst_fixed();
     /* (variant 8 of the FP64 path scans the cells and reads no sorted rows) */
     if (!EX && !(sizeof(R) == 8 && pst_var == 8))
       timed("rowsort", 3, [&] { Launch<D, R, EX>::rowsort(K, P, xs, pst_scratch, st); });

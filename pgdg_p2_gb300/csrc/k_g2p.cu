@@ -1924,18 +1924,30 @@ static void pst_d_launch(const CaseK& K, const DevPtrs<double>& P, int xs, int h
                                                                                                cap);
 }
 
-/* variants of the shifting kernel (the same members; results equal to rounding,
- * since variant 1 sums boundary particles in a second pass; the context's
- * autotuner times them on its own state and keeps the fastest): 0 per-lane row scan with
+/* variants of the shifting kernel (the same members, results equal to rounding:
+ * variant 1 sums boundary particles in a second pass, 6 and 7 work in packed pairs,
+ * 8 sums in cell order; on the mixed path the context's autotuner times them on
+ * its own state and keeps the fastest): 0 per-lane row scan with
  * queued members, 1 warp-cooperative row scan, 2 per-lane scan summing members
  * at once, 3 the same for 3 blocks per SM, 4 direct sums over bricks of twice
  * the cells with 512 threads, 5 over bricks of four times the cells with 1024
  * threads, 6 and 7 the second form (row-ordered records, global-row scan of
  * over-full bricks, packed pair arithmetic; 7 stages the records too).  The
- * exact path has one; 8, on the FP64_FMA path, is that kernel (k_pst_d). */
+ * exact path has one, k_pst_d, and the FP64_FMA path always takes the same kernel
+ * (8) unless told otherwise: it sums in another order than the rest, so a timed
+ * choice would let the bits depend on the clock, and it is the fastest at every size
+ * measured, with the row sort that the others need (ms per step, 8 against the best of
+ * 0 to 7: 24x11 cells 0.39 / 0.49, 112x48 0.33 / 0.42, 1024x1024 22.4 / 30.9, 40x10x10
+ * 2.84 / 4.56, 64x16x16 7.59 / 7.84, 192x48x48 128 / 195, and 108 / 144 with the
+ * shock in the bubble). */
+template <int D, typename R, bool EX>
+int Launch<D, R, EX>::pst_fixed() {
+  return EX ? 0 : sizeof(R) == 8 ? 8 : -1;
+}
+/* those that the mixed path's autotuner times */
 template <int D, typename R, bool EX>
 int Launch<D, R, EX>::pst_variants() {
-  return EX ? 1 : sizeof(R) == 8 ? 9 : 8; /* 8: k_pst_d on the FMA path */
+  return 8;
 }
 
 /* device scratch of the per-stage row sort (0 on the exact path) */
@@ -2002,6 +2014,7 @@ void Launch<D, R, EX>::pst(const CaseK& K, const DevPtrs<R>& P, int xs, int hs, 
                                       cudaStream_t);                                                       \
   template size_t Launch<D, R, EX>::pst_scratch_bytes(const CaseK&);                                       \
   template void Launch<D, R, EX>::rowsort(const CaseK&, const DevPtrs<R>&, int, void*, cudaStream_t);        \
+  template int Launch<D, R, EX>::pst_fixed(); \
   template int Launch<D, R, EX>::pst_variants();
 #ifdef PGDG_EXACT_TU
 PGDG_INST(2, double, true)

@@ -258,6 +258,7 @@ struct Launch {
   /* per-stage row sort the shifting kernel of the same stage reads (mixed and
    * FMA paths; no launch on the exact path) */
   static void rowsort(const CaseK&, const DevPtrs<R>&, int xs, void* scratch, cudaStream_t);
+  static int pst_fixed(); /* the variant that needs no timing, or -1 */
   static int pst_variants();
 };
 

@@ -155,7 +155,6 @@ struct Ctx : pgdg_ctx {
   double* d_tot = nullptr;
   IfaceQ Q{};
   int64_t q_room = 0; /* problems the queue's buffers hold (Q.cap: those a queued stage may use) */
-  PartScratch part;   /* root partition of the interface batch */
   unsigned char* pst_scratch = nullptr; /* per-stage row sort of the shifting kernel */
   /* every particle lies in its bucket's cell (true from binning until the
    * particles move); P2G then skips neighbour cells beyond its cut radius */
@@ -203,7 +202,6 @@ struct Ctx : pgdg_ctx {
     drop_graphs();
     for (auto e : ev_pool) cudaEventDestroy(e);
     for (void* p : allocs) cudaFree(p);
-    part.release();
     if (st) cudaStreamDestroy(st);
   }
 
@@ -950,7 +948,7 @@ struct Ctx : pgdg_ctx {
       const int rc = resize_queue(need, std::max(need, q_room));
       if (rc) return rc;
     }
-    const int rc = mgfm_seeded_reserve(net, part, Q.cap);
+    const int rc = mgfm_seeded_reserve(net, Q.cap);
     if (rc) err = "interface batch scratch: out of device memory";
     return rc;
   }
@@ -975,7 +973,7 @@ struct Ctx : pgdg_ctx {
       int rc = PGDG_OK;
       timed("mgfm_seeded", 1, [&] {
         rc = mgfm_seeded_run(nullptr, q.in6, q.mat, d_gam, d_pinf, K.mgfm_variant, q.out3, nullptr, q.cap,
-                             &P.cnt->mgfm_calls, part, st, q.tot + 1);
+                             &P.cnt->mgfm_calls, nullptr, st, q.tot + 1);
       });
       if (rc) return rc;
       q.phase = 2;
@@ -990,14 +988,14 @@ struct Ctx : pgdg_ctx {
      * 4.4 -> 3.6 ms per step, the same bits).  The batch's size stays on the device
      * (Q.tot): nothing is read back */
     if (iface_queue && !capturing) {
-      const int rc = mgfm_seeded_reserve(net, part, Q.cap);
+      const int rc = mgfm_seeded_reserve(net, Q.cap);
       if (rc) return rc;
     }
     timed("iface_gather", 3, [&] { Launch<D, R, EX>::iface_gather(K, P, Q, st); });
     int rc = PGDG_OK;
     timed("mgfm_seeded", net ? 3 : 1, [&] {
       rc = mgfm_seeded_run(net, Q.in6, Q.mat, d_gam, d_pinf, K.mgfm_variant, Q.out3, nullptr, Q.cap,
-                           &P.cnt->mgfm_calls, part, st, Q.tot + 1);
+                           &P.cnt->mgfm_calls, nullptr, st, Q.tot + 1);
     });
     if (rc) return rc;
     timed("grid_acc", 2, [&] { Launch<D, R, EX>::grid_acc_queued(K, P, Q, st); });
@@ -1432,7 +1430,7 @@ int pgdg_tune(pgdg_ctx* ctx, const char* kernel, int variant, int* chosen) {
 }
 int pgdg_set_iface_queue(pgdg_ctx* ctx, int on) {
   if (on && ctx->precision == PGDG_PREC_FP64) {
-    ctx->err = "the exact-order FP64 path solves interface problems inline";
+    ctx->err = "the exact-order FP64 path queues its interface problems by itself, and offers no other queue";
     return PGDG_EINVAL;
   }
   if (!on && ctx->net) {

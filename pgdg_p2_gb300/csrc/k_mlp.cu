@@ -807,9 +807,8 @@ int pgdg_mgfm_batched(const pgdg_mlp* net, const double* in6, const int8_t* mat2
   if (n < 0 || !in6 || !mat2 || !gam || !pinf || !out3 || nmat < 1) return PGDG_EINVAL;
   if (n == 0) return PGDG_OK;
   /* the partition scratch is the network's; plain solves need none */
-  PartScratch none;
   return mgfm_seeded_run((void*)net, in6, mat2, gam, pinf, variant, out3, iters, n, nullptr,
-                         net ? const_cast<pgdg_mlp*>(net)->part : none, 0, nullptr);
+                         net ? &const_cast<pgdg_mlp*>(net)->part : nullptr, 0, nullptr);
 }
 
 /* Seeds of pgdg_mgfm_batched_noalloc: a file-scope device array, so the call
@@ -878,24 +877,24 @@ void PartScratch::release() {
   cap = 0;
 }
 
-int mgfm_seeded_reserve(void* netv, PartScratch& ps, int64_t n) {
-  (void)ps; /* a stage's batch is not sorted */
+int mgfm_seeded_reserve(void* netv, int64_t n) {
   return netv ? static_cast<pgdg_mlp*>(netv)->reserve_seeds(n) : PGDG_OK;
 }
 
 int mgfm_seeded_run(void* netv, const double* in6, const int8_t* mat2, const double* gam, const double* pinf,
                     int variant, double* out3, int32_t* iters, int64_t n, unsigned long long* stats,
-                    PartScratch& ps, cudaStream_t st, const unsigned long long* dn) {
+                    PartScratch* ps, cudaStream_t st, const unsigned long long* dn) {
   if (n <= 0) return PGDG_OK;
   if (n > INT32_MAX) return PGDG_EINVAL;
   pgdg_mlp* m = static_cast<pgdg_mlp*>(netv);
   const double* sd = nullptr;
+  const int nt = newton_threads(n);
   if (m) {
     /* split seed path: features and baseline, the network, then Newton with the
      * seed formed per problem (same arithmetic as the fused k_seed) */
     const int rc = m->reserve_seeds(n);
     if (rc) return rc;
-    k_seed_features<<<g_for(n, newton_threads(n)), newton_threads(n), 0, st>>>(in6, mat2, gam, pinf, variant, m->Xb, m->seeds, m->sc, n, dn);
+    k_seed_features<<<g_for(n, nt), nt, 0, st>>>(in6, mat2, gam, pinf, variant, m->Xb, m->seeds, m->sc, n, dn);
     forward(m, m->Xb, m->Yb, n, st, dn);
     sd = m->seeds;
   }
@@ -906,22 +905,22 @@ int mgfm_seeded_run(void* netv, const double* in6, const int8_t* mat2, const dou
    * first: 2^22 problems 10.9 -> 5.9 ms; at 65537 217 us sorted and 242 unsorted, at
    * 1000 111 and 103.  A stage of a run (dn) is not sorted: nearly all its problems
    * have a root. */
-  const bool sorted = m && !dn && n > 16384;
+  const bool sorted = m && ps && !dn && n > 16384;
   if (!sorted) {
-    k_mgfm_seeded<<<g_for(n, newton_threads(n)), newton_threads(n), 0, st>>>(in6, mat2, gam, pinf, variant, sd, out3, iters, n, stats,
+    k_mgfm_seeded<<<g_for(n, nt), nt, 0, st>>>(in6, mat2, gam, pinf, variant, sd, out3, iters, n, stats,
                                                  m ? m->Yb : nullptr, m ? m->sc : nullptr, m ? m->d_params : nullptr,
                                                  nullptr, m && m->tc ? m->d_tcerr : nullptr, dn);
     return cudaGetLastError() == cudaSuccess ? PGDG_OK : PGDG_ECUDA;
   }
-  const int rc = ps.reserve(n);
+  const int rc = ps->reserve(n);
   if (rc) return rc;
   const unsigned long long nn = (unsigned long long)n;
-  cudaMemcpyAsync(ps.dn, &nn, sizeof(nn), cudaMemcpyHostToDevice, st);
-  k_root_flag<<<g_for(n, 256), 256, 0, st>>>(sd, ps.pos, n);
-  scan_u64(ps.pos, ps.blk, ps.dn, n, st);
-  k_root_perm<<<g_for(n, 256), 256, 0, st>>>(ps.pos, ps.blk + (n + 2047) / 2048, ps.perm, n);
-  k_mgfm_seeded<<<g_for(n, newton_threads(n)), newton_threads(n), 0, st>>>(in6, mat2, gam, pinf, variant, sd, out3, iters, n, stats,
-                                               m->Yb, m->sc, m->d_params, ps.perm, m->tc ? m->d_tcerr : nullptr, nullptr);
+  cudaMemcpyAsync(ps->dn, &nn, sizeof(nn), cudaMemcpyHostToDevice, st);
+  k_root_flag<<<g_for(n, 256), 256, 0, st>>>(sd, ps->pos, n);
+  scan_u64(ps->pos, ps->blk, ps->dn, n, st);
+  k_root_perm<<<g_for(n, 256), 256, 0, st>>>(ps->pos, ps->blk + (n + 2047) / 2048, ps->perm, n);
+  k_mgfm_seeded<<<g_for(n, nt), nt, 0, st>>>(in6, mat2, gam, pinf, variant, sd, out3, iters, n, stats,
+                                               m->Yb, m->sc, m->d_params, ps->perm, m->tc ? m->d_tcerr : nullptr, nullptr);
   return cudaGetLastError() == cudaSuccess ? PGDG_OK : PGDG_ECUDA;
 }
 }  // namespace pgdg

@@ -300,7 +300,7 @@ void alive_index(const int8_t* phase, unsigned long long* scan, unsigned long lo
 int mlp_tc_forward(const float* params, const float* X, float* Y, int64_t n, int* err, cudaStream_t st,
                    const unsigned long long* dn = nullptr);
 
-/* scratch of the root partition of a batch (prefix, block sums, order, count) */
+/* scratch of the root partition of a large seeded batch (prefix, block sums, order, count) */
 struct PartScratch {
   unsigned long long *pos = nullptr, *blk = nullptr, *dn = nullptr;
   int32_t* perm = nullptr;
@@ -311,13 +311,15 @@ struct PartScratch {
 /* seeded batched MGFM over device buffers (k_mlp.cu); stats += (calls,
  * iterations, cap hits).  Launches are sized for n; with dn the batch's live
  * count is *dn (clamped to n), read on the device, so the call reads nothing
- * back on the host and can be captured in a graph once its scratch holds n */
+ * back on the host and can be captured in a graph once the network's scratch
+ * holds n.  ps: the partition's scratch, not used (and may be NULL) with dn or
+ * without a network */
 int mgfm_seeded_run(void* net, const double* in6, const int8_t* mat2, const double* gam, const double* pinf,
                     int variant, double* out3, int32_t* iters, int64_t n, unsigned long long* stats,
-                    PartScratch& ps, cudaStream_t st, const unsigned long long* dn);
-/* allocate the scratch a batch of n needs (partition and, with a network, seeds
- * and features) ahead of a capture, so the captured call allocates nothing */
-int mgfm_seeded_reserve(void* net, PartScratch& ps, int64_t n);
+                    PartScratch* ps, cudaStream_t st, const unsigned long long* dn);
+/* allocate the scratch a stage's batch of n needs (a network's seeds and
+ * features) ahead of a capture, so the captured call allocates nothing */
+int mgfm_seeded_reserve(void* net, int64_t n);
 
 /* the synthetic workload id built in place on the device (k_case.cu): n
  * lattice particles and every cell, as the host builder makes them */

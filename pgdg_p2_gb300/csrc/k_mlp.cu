@@ -555,8 +555,9 @@ __global__ void k_root_perm(const unsigned long long* __restrict__ pos, const un
  * batch that is resident at once is the largest number of warps on any quarter, and
  * blocks of 64 spread it evenly; a larger batch wants all 2048 threads of an SM,
  * which the capped grid reaches with blocks of 256 (1000 problems: 86 us with 64,
- * 130 with 256; 65537: 228 and 257; 2^22: 13.1 ms and 11.8). */
-inline int newton_threads(int64_t n) { return n <= 152 * 1024 ? 64 : 256; }
+ * 130 with 256; 65537: 228 and 257; 2^22: 13.1 ms and 11.8).  A stage of a run knows
+ * its room, not its size, and its problems are few and come first, so it takes 64. */
+inline int newton_threads(int64_t n, bool stage = false) { return stage || n <= 152 * 1024 ? 64 : 256; }
 
 /* Newton from the seed (or the plain seed when seed is NULL or the entry is
  * negative); a seeded solve that has not converged at the cap is redone from
@@ -888,7 +889,7 @@ int mgfm_seeded_run(void* netv, const double* in6, const int8_t* mat2, const dou
   if (n > INT32_MAX) return PGDG_EINVAL;
   pgdg_mlp* m = static_cast<pgdg_mlp*>(netv);
   const double* sd = nullptr;
-  const int nt = newton_threads(n);
+  const int nt = newton_threads(n, dn != nullptr);
   if (m) {
     /* split seed path: features and baseline, the network, then Newton with the
      * seed formed per problem (same arithmetic as the fused k_seed) */

@@ -340,45 +340,79 @@ __device__ void set_split(const CaseK& K, const PState<D>& par, PState<D>& ch) {
 /* Split and merge are chains of short kernels, a few microseconds each whatever they
  * do on a small grid, so each does all that the slots' order allows: the flags and the
  * tiles' prefixes, the prefix over the tiles with the counters, the events with their
- * old neighbours, the lists with mark_in.  A split and four merge
- * passes, 6 and 7 launches each in place of 14: 112x48 cells 0.28 -> 0.15 ms per step,
- * 1024x1024 cells 0.65 -> 0.44, 384x96x96 cells 2.22 -> 2.08. */
-template <int D, typename R>
-__device__ __forceinline__ int split_code(const CaseK& K, const DevPtrs<R>& P, const R* X, int64_t p) {
-  P.target[p] = -1;
-  P.mflag[p] = 0;
-  if (P.phase[p] == 0) return 0;
-  double vol = (double)P.vol[p];
-  double x0 = (double)X[p];
-  if (vol > K.vol_max) return 1;
-  if (P.mark_in[p] == 1) {
-    double dp = root_d(vol, D);
-    if (dsub(x0, K.bl[0]) >= dp) return 2;
+ * old neighbours, the lists with mark_in.  A split and four merge passes, 6 and 7
+ * launches each in place of 14, ms per step: 112x48 cells 0.13 -> 0.03 (split) and
+ * 0.24 -> 0.12 (merge), 1024x1024 0.23 -> 0.12 and 0.43 -> 0.27, 96x24x24 0.078 -> 0.046
+ * and 0.30 -> 0.19, 384x96x96 0.77 -> 0.73 and 1.57 -> 1.08. */
+/* Ranks of a tile's events, scan[p] of a slot that has one, and their total, scan_blk.  Events
+ * are rare: a tile without any, and one past the last slot (a third of them in a context with
+ * room to grow), skips the prefix */
+template <typename R>
+__device__ __forceinline__ void tile_ranks(const DevPtrs<R>& P, int64_t p0, const unsigned long long (&v)[2]) {
+  unsigned long long total = 0ull;
+  if (__syncthreads_or(v[0] != 0ull || v[1] != 0ull)) {
+    const unsigned long long at = scan_1024(v[0] + v[1], &total);
+    if (v[0]) P.scan[p0] = at;
+    if (v[1]) P.scan[p0 + 1] = at + v[0];
   }
-  return x0 > K.br[0] ? 3 : 0;
+  if (threadIdx.x == 0) P.scan_blk[blockIdx.x] = total;
+}
+__device__ __forceinline__ bool past_last(unsigned long long* blk, int64_t n) {
+  if ((int64_t)blockIdx.x * SCAN_TILE < n) return false;
+  if (threadIdx.x == 0) blk[blockIdx.x] = 0ull;
+  return true;
+}
+/* a >= vol^(1/DIM), the inlet's test, decided in FP32 when a is more than 0.1% away (far
+ * beyond the rounding of either side): the exact root is some 100 FP64 operations, and the
+ * particles that need it stand in a few tiles, one after another on their SMs */
+template <int D>
+__device__ __forceinline__ bool past_root(double a, double vol) {
+  if (vol > 1e-30 && vol < 1e30) {
+    const float af = (float)a, rf = (D == 2) ? sqrtf((float)vol) : cbrtf((float)vol);
+    if (af > rf * 1.001f) return true;
+    if (af < rf * 0.999f) return false;
+  }
+  return a >= root_d(vol, D);
 }
 /* event of every slot; scan[p] of a slot that splits or enters receives its rank in
- * its tile (splits in the upper, inlets in the lower half), scan_blk the tile's total */
+ * its tile (splits in the upper, inlets in the lower half).
+ * A thread's loads go out together: one after another, each behind the test of the one
+ * before and the stores between, they were the kernel's time */
 template <int D, typename R>
 __global__ void __launch_bounds__(1024) k_split_flags(CaseK K, DevPtrs<R> P) {
   const int64_t n = (int64_t)P.cnt->n_slots;
+  if (past_last(P.scan_blk, n)) return;
   const R* X = P.X[P.xb];
   const int64_t p0 = (int64_t)blockIdx.x * SCAN_TILE + threadIdx.x * 2;
   unsigned long long v[2] = {0ull, 0ull};
+  bool live[2];
+  int8_t mark[2];
+  R vol[2], x0[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int64_t p = p0 + k < n ? p0 + k : 0;
+    live[k] = P.phase[p] != 0;
+    mark[k] = P.mark_in[p];
+    vol[k] = P.vol[p];
+    x0[k] = X[p];
+  }
 #pragma unroll
   for (int k = 0; k < 2; k++)
     if (p0 + k < n) {
-      const int code = split_code<D, R>(K, P, X, p0 + k);
+      int code = 0;
+      if (live[k]) {
+        if ((double)vol[k] > K.vol_max) code = 1;
+        else if (mark[k] == 1 && past_root<D>(dsub((double)x0[k], K.bl[0]), (double)vol[k])) code = 2;
+        else if ((double)x0[k] > K.br[0]) code = 3;
+      }
+      P.target[p0 + k] = -1;
+      P.mflag[p0 + k] = 0;
       if (code == 3) atomicAdd(&P.cnt->step_new, 1ull); /* outlet count (step_new reused) */
       if (code) atomicAdd(&P.cnt->split_events, 1ull);
       P.evcode[p0 + k] = (int8_t)code;
       v[k] = (code == 1) ? (1ull << 32) : (code == 2 ? 1ull : 0ull);
     }
-  unsigned long long total;
-  const unsigned long long at = scan_1024(v[0] + v[1], &total);
-  if (v[0]) P.scan[p0] = at;
-  if (v[1]) P.scan[p0 + 1] = at + v[0];
-  if (threadIdx.x == 0) P.scan_blk[blockIdx.x] = total;
+  tile_ranks(P, p0, v);
 }
 
 /* slots a merge pass sweeps: all, or none when the pass follows a pass of the same
@@ -599,9 +633,11 @@ __global__ void k_refresh3(CaseK K, DevPtrs<R> P, const unsigned long long* np, 
   const double lim = dmul(K.p_sz, 2.);
   const float lo2 = (float)(lim * lim * (1.0 - 1e-5)), hi2 = (float)(lim * lim * (1.0 + 1e-5));
   GRID_STRIDE(p, n) {
+    const bool aff = P.aff[p] != 0;
+    if (!mark && !aff) continue;
     const bool live = P.phase[p] != 0;
     if (mark && live) P.mark_in[p] = mark_of<D, R>(K, P, X, p);
-    if (!P.aff[p]) continue;
+    if (!aff) continue;
     P.aff[p] = 0;
     if (!live) continue;
     atomicAdd(&P.cnt->n_affected, 1ull);
@@ -727,6 +763,7 @@ __global__ void k_merge_a(CaseK K, DevPtrs<R> P, int chained) {
 template <int D, typename R>
 __global__ void __launch_bounds__(1024) k_merge_b(CaseK K, DevPtrs<R> P, int chained) {
   const int64_t n = (int64_t)merge_span(P.cnt, chained);
+  if (past_last(P.scan_blk, n)) return;
   const int64_t p0 = (int64_t)blockIdx.x * SCAN_TILE + threadIdx.x * 2;
   unsigned long long v[2] = {0ull, 0ull};
 #pragma unroll
@@ -740,11 +777,7 @@ __global__ void __launch_bounds__(1024) k_merge_b(CaseK K, DevPtrs<R> P, int cha
       v[k] = 1;
     }
   }
-  unsigned long long total;
-  const unsigned long long at = scan_1024(v[0] + v[1], &total);
-  if (v[0]) P.scan[p0] = at;
-  if (v[1]) P.scan[p0 + 1] = at + v[0];
-  if (threadIdx.x == 0) P.scan_blk[blockIdx.x] = total;
+  tile_ranks(P, p0, v);
 }
 
 /* Set_merge_ptcl (particle.cpp:614-661) + list fix-up (mpm.cpp:1637-1669) */

@@ -16,10 +16,16 @@ constexpr int BLK = 256;
 #define GRID_STRIDE(i, n) for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (n); \
                                i += (int64_t)gridDim.x * blockDim.x)
 
-/* threads per block of the per-cell kernels: blocks of 32 or 64 spread a grid of a
- * few thousand cells, whose time is the latency of one cell's chain, over all SMs
- * (blocks of 128 filled 42 of 152 at 112x48 cells) */
-inline int spread(int64_t n) { return n <= 152 * 8 * 32 ? 32 : n <= 152 * 8 * 64 ? 64 : 128; }
+/* threads per block of the per-cell kernels.  On the FP64 paths the FP64 pipe's chains are the
+ * time, and blocks of 32 or 64 spread a grid of a few thousand cells over more SMs (us per step
+ * with 32, 64 and 128; limiter 112x48 cells 265, 266, 278, residual 326, 326, 355; 48x12x12
+ * cells 543, 544, 568 and 1277, 1210, 1357; 80x20x20 773, 856, 861 and 3667, 3580, 3648).  In
+ * FP32 one wave of 128 is as fast or faster at every size (112x48 cells P2G 22.6, 22.0, 21.6,
+ * limiter 38.8, 36.5, 35.9; 96x24x24 P2G 92.6, 89.6, 88.1, learned residual 207, 214, 204) */
+template <typename R>
+inline int spread(int64_t n) {
+  return sizeof(R) == 4 ? 128 : n <= 152 * 8 * 32 ? 32 : n <= 152 * 8 * 64 ? 64 : 128;
+}
 
 template <int D>
 __device__ __forceinline__ void cijk(const CaseK& K, int64_t ci, int* idx) {
@@ -454,7 +460,7 @@ void Launch<D, R, EX>::p2g(const CaseK& K, const DevPtrs<R>& P, bool fresh_bins,
   const double hi = K.p_g * 1 * 3.2 / CUT_OFF;
   double hh = (D == 2) ? hi * hi : hi * hi * hi;
   double Cw = (D == 2) ? 1.0 / PI_REF / hh * 7. / 4. : 1.0 / PI_REF / hh * 21. / 16.;
-  k_p2g<D, R, EX><<<grid_for(K.ncell, spread(K.ncell)), spread(K.ncell), 0, st>>>(K, P, Cw, fresh_bins ? p2g_skip<D>(K) : 0);
+  k_p2g<D, R, EX><<<grid_for(K.ncell, spread<R>(K.ncell)), spread<R>(K.ncell), 0, st>>>(K, P, Cw, fresh_bins ? p2g_skip<D>(K) : 0);
 }
 
 /* the newly present phases k_p2g flagged (runs after it) */
@@ -463,7 +469,7 @@ void Launch<D, R, EX>::p2g_new(const CaseK& K, const DevPtrs<R>& P, cudaStream_t
   const double hi = K.p_g * 1 * 3.2 / CUT_OFF;
   double hh = (D == 2) ? hi * hi : hi * hi * hi;
   double Cw = (D == 2) ? 1.0 / PI_REF / hh * 7. / 4. : 1.0 / PI_REF / hh * 21. / 16.;
-  k_p2g_new<D, R, EX><<<grid_for(K.ncell, spread(K.ncell)), spread(K.ncell), 0, st>>>(K, P, Cw);
+  k_p2g_new<D, R, EX><<<grid_for(K.ncell, spread<R>(K.ncell)), spread<R>(K.ncell), 0, st>>>(K, P, Cw);
 }
 
 /* ------------------------------------------------------------------ */
@@ -680,7 +686,7 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(6)) k_limiter(CaseK K, D
 
 template <int D, typename R, bool EX>
 void Launch<D, R, EX>::limiter(const CaseK& K, const DevPtrs<R>& P, cudaStream_t st) {
-  k_limiter<D, R, EX><<<grid_for(K.ncell, spread(K.ncell)), spread(K.ncell), 0, st>>>(K, P);
+  k_limiter<D, R, EX><<<grid_for(K.ncell, spread<R>(K.ncell)), spread<R>(K.ncell), 0, st>>>(K, P);
 }
 
 /* ------------------------------------------------------------------ */
@@ -1204,7 +1210,7 @@ void Launch<D, R, EX>::grid_acc(const CaseK& K, const DevPtrs<R>& P, IfaceQ Q, c
   if (D == 3) voli = voli * K.ps[2];
   double ps[3] = {K.ps[0] / 2, K.ps[1] / 2, K.ps[2] / 2};
   double m1 = (ps[0] * ps[0] / 3.) * voli, m2 = (ps[1] * ps[1] / 3.) * voli, m3 = (ps[2] * ps[2] / 3.) * voli;
-  k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
+  k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
 }
 
 /* count, offsets and gather of the stage's interface problems, all on the
@@ -1218,8 +1224,8 @@ void Launch<D, R, EX>::iface_gather(const CaseK& K, const DevPtrs<R>& P, IfaceQ 
   const int nblk = scan_nblk(K.ncell + 1); /* with the end of the last cell */
   k_iface_ranks<D, R, EX><<<nblk, 1024, 0, st>>>(K, P, Q);
   k_iface_total<R, EX><<<1, 1024, 0, st>>>(Q, nblk);
-  if (Q.phase) k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
-  else k_grid_acc<D, R, EX, 2><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
+  if (Q.phase) k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
+  else k_grid_acc<D, R, EX, 2><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
 }
 
 template <int D, typename R, bool EX>
@@ -1229,9 +1235,9 @@ void Launch<D, R, EX>::grid_acc_queued(const CaseK& K, const DevPtrs<R>& P, Ifac
   if (D == 3) voli = voli * K.ps[2];
   double ps[3] = {K.ps[0] / 2, K.ps[1] / 2, K.ps[2] / 2};
   double m1 = (ps[0] * ps[0] / 3.) * voli, m2 = (ps[1] * ps[1] / 3.) * voli, m3 = (ps[2] * ps[2] / 3.) * voli;
-  k_grid_acc<D, R, EX, 3><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
+  k_grid_acc<D, R, EX, 3><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
   /* the inline solve of a stage that outgrew the queue (returns at once otherwise) */
-  k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread(nth)), spread(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
+  k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
 }
 
 /* ------------------------------------------------------------------ */
@@ -1328,7 +1334,7 @@ __global__ void __launch_bounds__(256) k_update_grid(CaseK K, DevPtrs<R> P, int 
 
 template <int D, typename R, bool EX>
 void Launch<D, R, EX>::update_grid(const CaseK& K, const DevPtrs<R>& P, int md, cudaStream_t st) {
-  k_update_grid<D, R, EX><<<grid_for(K.ncell, spread(K.ncell)), spread(K.ncell), 0, st>>>(K, P, md);
+  k_update_grid<D, R, EX><<<grid_for(K.ncell, spread<R>(K.ncell)), spread<R>(K.ncell), 0, st>>>(K, P, md);
 }
 
 /* ------------------------------------------------------------------ */

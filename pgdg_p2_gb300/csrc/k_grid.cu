@@ -20,11 +20,16 @@ constexpr int BLK = 256;
  * time, and blocks of 32 or 64 spread a grid of a few thousand cells over more SMs (us per step
  * with 32, 64 and 128; limiter 112x48 cells 265, 266, 278, residual 326, 326, 355; 48x12x12
  * cells 543, 544, 568 and 1277, 1210, 1357; 80x20x20 773, 856, 861 and 3667, 3580, 3648).  In
- * FP32 one wave of 128 is as fast or faster at every size (112x48 cells P2G 22.6, 22.0, 21.6,
- * limiter 38.8, 36.5, 35.9; 96x24x24 P2G 92.6, 89.6, 88.1, learned residual 207, 214, 204) */
+ * FP32 blocks of 128 are as fast or faster (112x48 cells P2G 22.6, 22.0, 21.6, limiter 38.8,
+ * 36.5, 35.9; 96x24x24 P2G 92.6, 89.6, 88.1, learned residual 207, 214, 204), but for the inline
+ * residual in its second wave (two blocks of 128 an SM: 38,912 cells a wave), whose rest 64
+ * spread better (332x142 cells 71.6 + 82 of 64, 71.2 + 90 of 128; 400x170 85 + 125 and 97 + 139;
+ * earlier, 300x128, 69 + 75.6 and 69 + 74; later, 160x40x40, 136 + 426 and 136 + 404) */
 template <typename R>
-inline int spread(int64_t n) {
-  return sizeof(R) == 4 ? 128 : n <= 152 * 8 * 32 ? 32 : n <= 152 * 8 * 64 ? 64 : 128;
+inline int spread(int64_t n, bool inline_residual = false) {
+  constexpr int64_t wave = 152 * 8 * 32;
+  if (sizeof(R) == 4) return inline_residual && n > wave && n <= 2 * wave ? 64 : 128;
+  return n <= wave ? 32 : n <= 2 * wave ? 64 : 128;
 }
 
 template <int D>
@@ -1210,7 +1215,7 @@ void Launch<D, R, EX>::grid_acc(const CaseK& K, const DevPtrs<R>& P, IfaceQ Q, c
   if (D == 3) voli = voli * K.ps[2];
   double ps[3] = {K.ps[0] / 2, K.ps[1] / 2, K.ps[2] / 2};
   double m1 = (ps[0] * ps[0] / 3.) * voli, m2 = (ps[1] * ps[1] / 3.) * voli, m3 = (ps[2] * ps[2] / 3.) * voli;
-  k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
+  k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread<R>(nth, true)), spread<R>(nth, true), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
 }
 
 /* count, offsets and gather of the stage's interface problems, all on the
@@ -1224,7 +1229,7 @@ void Launch<D, R, EX>::iface_gather(const CaseK& K, const DevPtrs<R>& P, IfaceQ 
   const int nblk = scan_nblk(K.ncell + 1); /* with the end of the last cell */
   k_iface_ranks<D, R, EX><<<nblk, 1024, 0, st>>>(K, P, Q);
   k_iface_total<R, EX><<<1, 1024, 0, st>>>(Q, nblk);
-  if (Q.phase) k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
+  if (Q.phase) k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread<R>(nth, true)), spread<R>(nth, true), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
   else k_grid_acc<D, R, EX, 2><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, 0, 0, 0, Q);
 }
 

@@ -1631,7 +1631,7 @@ static void pst2_launch(const CaseK& K, const DevPtrs<R>& P, int xs, int hs, int
 }
 
 /* ---- the shifting kernel of the FP64 paths ----
- * An FP64 instruction occupies a quarter of an SM for 64 cycles a warp, 32 times
+ * An FP64 instruction occupies a quarter of an SM for 64 cycles a warp, 64 times
  * an FP32 one, so everything that only decides is done in FP32: positions are
  * staged relative to the brick's centre as (x, y, z, slot) in 16 bytes, cells
  * are pruned by their FP32 bounds, and a candidate is a member or not by its FP32

@@ -555,7 +555,7 @@ __global__ void k_root_perm(const unsigned long long* __restrict__ pos, const un
  * batch that is resident at once is the largest number of warps on any quarter, and
  * blocks of 64 spread it evenly; a larger batch wants all 2048 threads of an SM,
  * which the capped grid reaches with blocks of 256 (1000 problems: 86 us with 64,
- * 130 with 256; 65537: 228 and 257; 2^22: 13.1 ms and 11.8).  A stage of a run knows
+ * 130 with 256; 65537: 235 and 257; 2^22: 13.1 ms and 11.8).  A stage of a run knows
  * its room, not its size, and its problems are few and come first, so it takes 64. */
 inline int newton_threads(int64_t n, bool stage = false) { return stage || n <= 152 * 1024 ? 64 : 256; }
 
@@ -901,7 +901,7 @@ int mgfm_seeded_run(void* netv, const double* in6, const int8_t* mat2, const dou
   }
   /* A problem without a root takes about as long as one with a root from the plain
    * seed (mgfm replays its descent), so plain solves are one launch: 2^22 problems
-   * 17.3 -> 11.8 ms, 65537 problems 550 -> 255 us.  Seeded, it takes about six
+   * 17.3 -> 11.8 ms, 65537 problems 495 -> 235 us.  Seeded, it takes about six
    * iterations and the others two, and a batch is sorted, problems with a root
    * first: 2^22 problems 10.9 -> 5.9 ms; at 65537 217 us sorted and 242 unsorted, at
    * 1000 111 and 103.  A stage of a run (dn) is not sorted: nearly all its problems

@@ -1644,9 +1644,9 @@ static void pst2_launch(const CaseK& K, const DevPtrs<R>& P, int xs, int hs, int
  * full, mostly once: queues of 64, emptied at 32, left 13.5 of 32 lanes active in
  * the pair terms.  Bricks of 8 (3D) or 16 (2D) cells, 64 threads: small enough
  * that a few thousand cells still fill the chip evenly.
- * Exact path, shifting per step: 48x12x12 cells 13.1 -> 7.7 ms (73 % of the FP64
+ * Exact path, shifting per step: 48x12x12 cells 13.1 -> 7.8 ms (73 % of the FP64
  * pipe's issue slots in the SMs at work), 112x48 1.19 -> 0.58 ms; FMA path 200x200
- * 1.48 -> 1.15 ms, 112x48 0.366 -> 0.332, 64x16x16 7.66 -> 7.64. */
+ * 1.48 -> 1.15 ms, 112x48 0.366 -> 0.332 (and no row sort: see the variants below). */
 template <int D>
 struct SmallBrick;
 template <>

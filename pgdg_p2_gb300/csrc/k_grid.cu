@@ -731,11 +731,21 @@ __device__ __forceinline__ void flux_col(const R* Uu, const R* v, R Pp, int a, R
 
 /* lanes per cell of the residual: on the FP64 paths a lane takes one face (and one
  * the volume integral), since one cell is a chain of 16,000 dependent FP64
- * instructions (48x12x12 cells: 1.51 ms per launch with a thread per cell, 0.60
- * with eight); the lanes' parts are added in the order of the serial loop */
+ * instructions; the lanes' parts are added in the order of the serial loop */
 template <typename R>
 __host__ __device__ constexpr int acc_lanes() {
   return sizeof(R) == 8 ? 8 : 1;
+}
+/* Up to which grid the FP64 residual spreads its cells over lanes.  Faces and volume integral run
+ * one after another in a warp whichever of its lanes want them, so eight lanes issue 2 (2D) or
+ * 1.3 (3D) times the face work and 8 times the volume's: once the chip has warps enough with a
+ * thread a cell, the FP64 pipe is the time and that form is faster (exact path, us per step with
+ * one thread and with eight: 168x72 cells 628 and 555, 128x128 683 and 712, 256x256 1281 and
+ * 2396, 512x512 3522 and 9248; 64x16x16 3156 and 1964, 80x20x20 3709 and 3760, 96x24x24 4453
+ * and 6033, 160x40x40 13634 and 25849) */
+template <int D>
+inline bool acc_spread(int64_t ncell) {
+  return ncell <= (D == 3 ? 152 * 208 : 152 * 96);
 }
 /* interface problems of cell idx's phase ss on face f */
 template <int D, typename R>
@@ -753,7 +763,7 @@ __device__ __forceinline__ int face_problems(const CaseK& K, const int* idx, int
 
 /* MODE 0: MGFM solved inline (FP32: or gathered and used, see phase); MODE 2: queue every interface problem (no flux
  * work); MODE 3: read the ghost states of the interface problems from the queue */
-template <int D, typename R, bool EX, int MODE>
+template <int D, typename R, bool EX, int MODE, int G = acc_lanes<R>()>
 __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_grid_acc(CaseK K, DevPtrs<R> P, int variant, double voli_d,
                                                  double mij1, double mij2, double mij3, IfaceQ Q) {
   constexpr int U = D + 2, B = D + 1, NF = 2 * D, NQ = (D == 3) ? 4 : 2, NG = (D == 3) ? 8 : 4;
@@ -777,7 +787,6 @@ __global__ void __launch_bounds__(128, minblocks_f32<R>(MODE == 0 ? 2 : 3)) k_gr
    * problems and residual round as in the inline solve */
   constexpr bool PH = MODE == 0 && sizeof(R) == 4;
   const int phase = PH ? Q.phase : 0;
-  constexpr int G = acc_lanes<R>();
   const int sub = (int)threadIdx.x & (G - 1);
   const unsigned gmask = G == 1 ? 0u : 0xffu << (threadIdx.x & 24);
   __shared__ R s_part[G == 1 ? 1 : 128 / G][G == 1 ? 1 : NF + 1][G == 1 ? 1 : U * B];
@@ -1240,7 +1249,10 @@ void Launch<D, R, EX>::grid_acc_queued(const CaseK& K, const DevPtrs<R>& P, Ifac
   if (D == 3) voli = voli * K.ps[2];
   double ps[3] = {K.ps[0] / 2, K.ps[1] / 2, K.ps[2] / 2};
   double m1 = (ps[0] * ps[0] / 3.) * voli, m2 = (ps[1] * ps[1] / 3.) * voli, m3 = (ps[2] * ps[2] / 3.) * voli;
-  k_grid_acc<D, R, EX, 3><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
+  if (sizeof(R) == 8 && !acc_spread<D>(K.ncell))
+    k_grid_acc<D, R, EX, 3, 1><<<grid_for(K.ncell, spread<R>(K.ncell)), spread<R>(K.ncell), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
+  else
+    k_grid_acc<D, R, EX, 3><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
   /* the inline solve of a stage that outgrew the queue (returns at once otherwise) */
   k_grid_acc<D, R, EX, 0><<<grid_for(nth, spread<R>(nth)), spread<R>(nth), 0, st>>>(K, P, K.mgfm_variant, voli, m1, m2, m3, Q);
 }
